@@ -48,7 +48,9 @@ extern "C" {
 #define JNE_ERR_FORMAT 7  /* not an EIGENVALS_V6 file, or inconsistent records */
 
 /* arithmetic of the Gram contraction */
-#define JNE_PREC_FP64 0  /* plain FP64 fused kernel */
+/* plain form: exact Gram sums (digits of the engine's increments on the tensor
+ * cores; FP64 multiply-adds for explicit increments), FP64 record and solve */
+#define JNE_PREC_FP64 0
 #define JNE_PREC_MIXED 1 /* split FP16/TF32 tensor-core Grams, FP32 chunks, float-float merge, FP64 solve */
 /* JNE_PREC_MIXED requests with fewer steps than this run the FP64 kernel: on
  * such short paths the FP32 chunk part is most of every moment. */
@@ -130,9 +132,8 @@ int jne_eigs_seeded(jne_context* ctx, int model, int dim, int steps, uint64_t ba
 
 /* As jne_eigs_seeded, with out in device memory, enqueued asynchronously:
  * work later enqueued on `stream` (a cudaStream_t; null = the context's
- * stream) sees the results, and the call returns without waiting.  Consecutive
- * calls overlap (the finalize of one batch runs beside the accumulation of the
- * next).  Device-side errors (a non-SPD S11) are reported by jne_sync. */
+ * stream) sees the results, and the call returns without waiting.  Device-side
+ * errors (a non-SPD S11) are reported by jne_sync. */
 int jne_eigs_seeded_device(jne_context* ctx, int model, int dim, int steps, uint64_t base_seed,
                            uint32_t seed_first, int64_t n_runs, int precision, double* out_device, void* stream);
 
@@ -151,7 +152,7 @@ int jne_eigs_seeded_models(jne_context* ctx, const int* models, int n_models, in
  * cannot allocate device memory -- a host framework that owns the GPU's
  * allocator and forbids foreign allocations, a real-time loop that allows no
  * allocation after start-up.  It needs no context: its scratch (the moment
- * records, the chunk and entry tables, the counters and the status word) is one
+ * records, the chunk table, the counters and the status word) is one
  * file-scope __device__ array of JNE_NOALLOC_SCRATCH_BYTES (4.7 MiB) that every
  * GPU loading this library holds until the process exits, and it calls no
  * cudaMalloc, cudaFree or allocating library routine.  It runs the kernels and

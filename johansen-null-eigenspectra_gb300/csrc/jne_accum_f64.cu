@@ -1,16 +1,18 @@
-// jne_accum_f64.cu -- plain FP64 fused accumulation: one warp per run.
+// jne_accum_f64.cu -- FP64 accumulation of explicit increments: one warp per run.
 //
-// Replaces, per run, the work of rng_matrix.rs:57-141 (Gaussian path),
-// johansen_statistics.rs:102-197 (F construction) and the two
-// sum_of_outer_products calls of johansen_statistics.rs:32-33: instead of
-// materialising B and F, each run accumulates in FP64 exactly the raw moments
-// its model needs (listed in a per-(model, dim) entry table), from which the
-// finalize kernel rebuilds S11 and S10.
+// Replaces, per run, the work of johansen_statistics.rs:102-197 (F
+// construction) and the two sum_of_outer_products calls of
+// johansen_statistics.rs:32-33: instead of materialising B and F, each run
+// accumulates in FP64 multiply-adds the raw moments its model needs (listed in a
+// per-(model, dim) entry table), from which the finalize kernel rebuilds S11 and
+// S10.  The engine's own increments take jne_accum_digits.cuh, whose fixed-point
+// grid an arbitrary FP64 increment does not fit.
 //
-// Per 32-step tile: lane t draws the increments of column t0+t (Philox), the
-// first d lanes run the FP64 walk along time, and every lane adds its <= MAXE
-// table entries sum_t v_t[a] * v_t[b] over the tile, where
-// v_t = [W_0..W_{d-1}, z_0..z_{d-1}, 1, y, y^2, 0].  Nothing T-sized touches HBM.
+// Per 32-step tile: lane t reads the increments of column t0+t, the first d
+// lanes run the FP64 walk along time, and every lane adds its <= MAXE table
+// entries sum_t v_t[a] * v_t[b] over the tile, where
+// v_t = [W_0..W_{d-1}, z_0..z_{d-1}, 1, y, y^2, 0].  Bound by the FP64 pipe (64
+// cycles a warp instruction and scheduler).
 #include "jne_common.cuh"
 #include "jne_kernels.h"
 
@@ -18,7 +20,7 @@ namespace {
 
 constexpr int kF64Warps = 4;  // warps per block
 
-template <int MAXE, bool EXT>
+template <int MAXE>
 __global__ void __launch_bounds__(kF64Warps * JNE_WARP)
     k_accum_f64(const jne_accum_args a, const int4* __restrict__ ent, const int nent) {
   extern __shared__ double smem[];
@@ -41,36 +43,21 @@ __global__ void __launch_bounds__(kF64Warps * JNE_WARP)
     }
   }
   const double invT = 1.0 / (double)T;
-  const int nq = (d + 3) >> 2;
-  const jne_round_keys rk = jne_make_round_keys(a.key0, a.key1);
   const int nwarps = gridDim.x * kF64Warps;
   __syncwarp();
 
   for (int run = blockIdx.x * kF64Warps + wib; run < a.n_runs; run += nwarps) {
-    const uint32_t seed = a.seed_first + (uint32_t)run;
     double acc[MAXE];
 #pragma unroll
     for (int m = 0; m < MAXE; m++) acc[m] = 0.0;
     double carry = 0.0;  // lane f < d: W_f at the tile start
 
     for (int t0 = 0; t0 < T; t0 += JNE_WARP) {
-      const int i = t0 + lane;  // column i draws step s = i + 1
+      const int i = t0 + lane;
       const bool valid = i < T;
       double* vr = v + lane * VS;
-      if (EXT) {
-        const double* src = a.ext + ((size_t)run * T + (valid ? i : 0)) * d;
-        for (int f = 0; f < d; f++) vr[d + f] = valid ? src[f] : 0.0;
-      } else {
-        for (int j = 0; j < nq; j++) {
-          float z[4];
-          jne_normal_quad((uint32_t)(i + 1), (uint32_t)j, seed, rk, z);
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int f = 4 * j + e;
-            if (f < d) vr[d + f] = valid ? (double)z[e] : 0.0;
-          }
-        }
-      }
+      const double* src = a.ext + ((size_t)run * T + (valid ? i : 0)) * d;
+      for (int f = 0; f < d; f++) vr[d + f] = valid ? src[f] : 0.0;
       const double y = (double)(i + 1) * invT;
       vr[2 * d] = valid ? 1.0 : 0.0;
       vr[2 * d + 1] = valid ? y : 0.0;
@@ -106,7 +93,7 @@ cudaError_t launch_maxe(const jne_accum_args& a, const int4* ent, int nent, int 
   const int VS = 2 * a.dim + 5;
   const size_t shm = (size_t)kF64Warps * JNE_WARP * VS * sizeof(double);
   const int threads = kF64Warps * JNE_WARP;
-  auto k = a.ext ? k_accum_f64<MAXE, true> : k_accum_f64<MAXE, false>;
+  auto k = k_accum_f64<MAXE>;
   // persistent grid: the resident blocks, so every warp strides over the same number of runs
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, shm) != cudaSuccess || per_sm < 1)
@@ -121,6 +108,7 @@ cudaError_t launch_maxe(const jne_accum_args& a, const int4* ent, int nent, int 
 
 cudaError_t jne_launch_accum_f64(const jne_accum_args& a, const int4* ent, int nent, int sms, cudaStream_t st) {
   if (a.n_runs <= 0) return cudaSuccess;
+  if (!a.ext) return cudaErrorInvalidValue;
   switch ((nent + JNE_WARP - 1) / JNE_WARP) {
     case 1: return launch_maxe<1>(a, ent, nent, sms, st);
     case 2: return launch_maxe<2>(a, ent, nent, sms, st);
@@ -135,15 +123,14 @@ cudaError_t jne_launch_accum_f64(const jne_accum_args& a, const int4* ent, int n
   }
 }
 
-// Entry table of a (model, dim) pair; model < 0 requests the union of all
-// five models (every slot except Nz1, which comes from the walk's end point).
+// Entry table of a (model, dim) pair: the moments its F needs (Nz1 comes from the
+// walk's end point).
 int jne_build_f64_entries(int model, int d, int4* out, int cap) {
   const int W = 0, Z = d, ONE = 2 * d, Y = 2 * d + 1, YY = 2 * d + 2;
-  const bool all = model < 0;
-  const int nb = (!all && (model == 2 || model == 4)) ? d - 1 : d;  // walk rows entering F
-  const bool need_w1 = all || model >= 1;
-  const bool need_y = all || model >= 2;
-  const bool need_yy = all || model == 4;
+  const int nb = (model == 2 || model == 4) ? d - 1 : d;  // walk rows entering F
+  const bool need_w1 = model >= 1;
+  const bool need_y = model >= 2;
+  const bool need_yy = model == 4;
   int n = 0;
   auto put = [&](int x, int y, int s) {
     if (n < cap) out[n] = make_int4(x, y, s, 0);

@@ -34,13 +34,8 @@ int jne_open(int device, unsigned long long mem_budget_bytes, jne_context** out)
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->fin_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
-  for (int i = 0; i < 2 && e == cudaSuccess; i++) {
-    e = cudaEventCreateWithFlags(&c->ev_acc[i], cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fin[i], cudaEventDisableTiming);
-  }
+  for (int i = 0; i < 2 && e == cudaSuccess; i++) e = cudaEventCreateWithFlags(&c->ev_fin[i], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_status, sizeof(unsigned int));
   // the asynchronous paths only clear the status in jne_sync: start from zero
   if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, sizeof(unsigned int));
@@ -57,7 +52,6 @@ int jne_open(int device, unsigned long long mem_budget_bytes, jne_context** out)
 void jne_close(jne_context* c) {
   if (!c) return;
   cudaSetDevice(c->device);
-  if (c->fin_stream) cudaStreamSynchronize(c->fin_stream);
   if (c->stream) cudaStreamSynchronize(c->stream);
   prof_flush(c);
   for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
@@ -73,7 +67,6 @@ void jne_close(jne_context* c) {
   cudaFree(c->d_batch);
   cudaFree(c->d_qscratch);
   if (c->ev_in) cudaEventDestroy(c->ev_in);
-  if (c->ev_join) cudaEventDestroy(c->ev_join);
   for (int i = 0; i < 2; i++) {
     cudaFree(c->d_sink[i]);
     cudaFree(c->d_sink_st[i]);
@@ -89,10 +82,8 @@ void jne_close(jne_context* c) {
     cudaFreeHost(c->h_reqs[i]);
     cudaFreeHost(c->h_rtab[i]);
     cudaFree(c->d_momb[i]);
-    if (c->ev_acc[i]) cudaEventDestroy(c->ev_acc[i]);
     if (c->ev_fin[i]) cudaEventDestroy(c->ev_fin[i]);
   }
-  if (c->fin_stream) cudaStreamDestroy(c->fin_stream);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -176,8 +167,6 @@ int jne_eigs_seeded_models(jne_context* c, const int* models, int n_models, int 
   for (int m = 0; m < n_models; m++) k_total += jne_eigen_count(models[m], dim);
   uint32_t k0, k1;
   stream_key(base_seed, dim, &k0, &k1);
-  // a single FP64 pass needs every moment any requested model uses
-  const int acc_model = (n_models == 1) ? models[0] : -1;
   cudaStream_t st = c->stream;
   int rc = drain(c);
   if (rc) return rc;
@@ -192,7 +181,7 @@ int jne_eigs_seeded_models(jne_context* c, const int* models, int n_models, int 
     // (finalizing five models per batch inside the accumulation stalls its warps longer than the
     // separate kernels take: 0.14 s against 0.08 s for 5 x 200k runs)
     const jne_finalize_args f0 = finalize_args(c, models[0], dim, steps, n, c->d_mom, c->d_out);
-    if ((rc = accumulate(c, acc_model, dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
+    if ((rc = accumulate(c, models[0], dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
                          c->d_mom, st, n_models == 1 ? &f0 : nullptr)))
       return rc;
     size_t off = 0;
@@ -232,8 +221,7 @@ int jne_eigs_seeded_device(jne_context* c, int model, int dim, int steps, uint64
 int jne_sync(jne_context* c) {
   if (!c) return JNE_ERR_ARG;
   if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, JNE_ERR_CUDA, "cudaSetDevice failed");
-  cudaError_t e = cudaStreamSynchronize(c->fin_stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaError_t e = cudaStreamSynchronize(c->stream);
   unsigned int stv = 0;
   if (e == cudaSuccess) e = cudaMemcpy(&stv, c->d_status, sizeof(stv), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, sizeof(unsigned int));

@@ -161,14 +161,13 @@ int jne_detail::run_batch(jne_context* c, const jne_request* reqs, int n_req, do
     if ((rc = check_request(c, reqs[i], outs[i]))) return rc;
   if ((rc = join_in(c, user))) return rc;
   int last = -1;
-  bool seeded = false;  // some request finalizes on the context's second stream
   std::vector<int> ragged;
   for (int i = 0; i < n_req; i++) {
     if (reqs[i].n_runs == 0) continue;
     if (ragged_ok(reqs[i])) {
       ragged.push_back(i);
-    } else if (seeded = true, (rc = enqueue_seeded(c, reqs[i].model, reqs[i].dim, reqs[i].steps, reqs[i].base_seed,
-                                    reqs[i].seed_first, reqs[i].n_runs, reqs[i].precision, outs[i], &last,
+    } else if ((rc = enqueue_seeded(c, reqs[i].model, reqs[i].dim, reqs[i].steps, reqs[i].base_seed, reqs[i].seed_first,
+                                    reqs[i].n_runs, reqs[i].precision, outs[i], &last,
                                     req_status ? req_status[i] : nullptr))) {
       return rc;
     }
@@ -217,11 +216,6 @@ int jne_detail::run_batch(jne_context* c, const jne_request* reqs, int n_req, do
     c->fin_pending[b] = true;
     last = b;
   }
-  // the caller's stream waits for both streams' work: the ragged launches (the
-  // last one's event) and the FP64-path finalizes queued on the second stream
-  if (seeded && ((e = cudaEventRecord(c->ev_join, c->fin_stream)) != cudaSuccess ||
-                 (e = cudaStreamWaitEvent(user, c->ev_join, 0)) != cudaSuccess))
-    return cuda_fail(c, e, "stream join");
   return join_out(c, user, last);
 }
 
@@ -395,7 +389,6 @@ int jne_run_batch_sink(jne_context* c, const jne_request* reqs, int n_req, const
   }
   if (rc) {
     cudaStreamSynchronize(st);  // no round left writing into the slots
-    cudaStreamSynchronize(c->fin_stream);
     return rc;
   }
   if (worst != JNE_OK) return fail(c, worst, "some runs of the batch had a non-SPD S11 (NaN rows delivered)");

@@ -51,15 +51,13 @@ struct jne_context {
   unsigned long long* d_qscratch = nullptr;  // percentile analyzer: keys, ranks, histograms
   size_t qscratch_cap = 0;
   std::string err;
-  // asynchronous device path: two record buffers, finalize on a second stream
-  cudaStream_t fin_stream = nullptr;
-  cudaEvent_t ev_acc[2] = {nullptr, nullptr}, ev_fin[2] = {nullptr, nullptr};
+  // asynchronous device path: two record buffers, each with the event of its last launch
+  cudaEvent_t ev_fin[2] = {nullptr, nullptr};
   bool fin_pending[2] = {false, false};
   double* d_momb[2] = {nullptr, nullptr};
   size_t momb_cap[2] = {0, 0};
   unsigned long long batch_seq = 0;
-  cudaEvent_t ev_in = nullptr;    // joins a caller's stream into the context's streams
-  cudaEvent_t ev_join = nullptr;  // the finalize stream's work of a batch -> the caller's stream
+  cudaEvent_t ev_in = nullptr;  // joins a caller's stream into the context's
   // ragged batches: per record buffer, the device request table, chunk tables,
   // work counter, and pinned host staging for the tables
   jne_ragged_req* d_reqs[2] = {nullptr, nullptr};
@@ -306,9 +304,9 @@ inline jne_finalize_args finalize_args(jne_context* c, int model, int dim, int s
 }
 
 // Moments of runs [seed_first, seed_first + n) into mom (leading dim n).  With
-// `fin`, the runs' eigenvalues are also produced on st: inside the mixed
-// kernel (each warp finalizes its runs), or by a finalize launch after the
-// FP64 kernel.  The accumulation's status bits go to `status` (null: the
+// `fin`, the runs' eigenvalues are also produced on st: inside the kernel (each
+// warp finalizes its runs), or by a finalize launch after the FP64 kernel of
+// explicit increments.  The accumulation's status bits go to `status` (null: the
 // context's status word).
 inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t key0, uint32_t key1, uint32_t seed_first,
                       int n, int precision, const double* d_ext, double* mom, cudaStream_t st,
@@ -329,7 +327,7 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
   a.mom_ld = n;
   a.status = status ? status : c->d_status;
   cudaError_t e;
-  if (precision == JNE_PREC_FP64) {
+  if (precision == JNE_PREC_FP64 && d_ext) {  // explicit increments: FP64 multiply-adds
     if (c->ent_model != model || c->ent_dim != dim) {
       int4 host_ent[512];
       c->ent_n = jne_build_f64_entries(model, dim, host_ent, 512);
@@ -340,46 +338,46 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
       c->ent_model = model;
       c->ent_dim = dim;
     }
-    const int nent = c->ent_n;
     {
       ProfScope ps(c, JNE_KERNEL_ACCUM_FP64, st);
-      e = jne_launch_accum_f64(a, c->d_ent, nent, c->sms, st);
+      e = jne_launch_accum_f64(a, c->d_ent, c->ent_n, c->sms, st);
     }
     if (e != cudaSuccess) return cuda_fail(c, e, "accumulation launch");
     return fin ? finalize(c, *fin, st) : JNE_OK;
-  } else {
+  }
+  if (precision == JNE_PREC_MIXED) {
     // per-chunk time means, exact (integer sums) then rounded once
     const int nch = (steps + a.chunk - 1) / a.chunk;
     if (c->ctab_steps != steps || c->ctab_chunk != a.chunk) {
-    int rc = ensure(c, &c->d_ctab, &c->ctab_cap, (size_t)nch, "chunk table");
-    if (rc) return rc;
-    c->h_ctab.resize(nch);
-    fill_chunk_table(steps, a.chunk, c->h_ctab.data());
-    e = cudaMemcpyAsync(c->d_ctab, c->h_ctab.data(), sizeof(jne_chunk_time) * nch, cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return cuda_fail(c, e, "chunk table upload");
-    c->ctab_steps = steps;
-    c->ctab_chunk = a.chunk;
+      int rc = ensure(c, &c->d_ctab, &c->ctab_cap, (size_t)nch, "chunk table");
+      if (rc) return rc;
+      c->h_ctab.resize(nch);
+      fill_chunk_table(steps, a.chunk, c->h_ctab.data());
+      e = cudaMemcpyAsync(c->d_ctab, c->h_ctab.data(), sizeof(jne_chunk_time) * nch, cudaMemcpyHostToDevice, st);
+      if (e != cudaSuccess) return cuda_fail(c, e, "chunk table upload");
+      c->ctab_steps = steps;
+      c->ctab_chunk = a.chunk;
     }
     a.chunk_tab = c->d_ctab;
     const jne_shape shape = shape_for(c, dim, steps);
     a.blocks_per_sm = d_ext ? 4 : shape.blocks_per_sm;
     a.pack = d_ext || shape.pack ? 0 : -1;
-    // warps take runs from a counter, so blocks that start late (behind a
-    // concurrent finalize) take fewer runs instead of leaving a tail
-    e = cudaMemsetAsync(c->d_next_run, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return cuda_fail(c, e, "work counter reset");
-    a.next_run = c->d_next_run;
-    if (fin) {
-      const size_t nb = ((size_t)n + 31) / 32;
-      int rc = ensure(c, &c->d_batch, &c->batch_cap, nb, "batch counts");
-      if (rc) return rc;
-      e = cudaMemsetAsync(c->d_batch, 0, sizeof(unsigned int) * nb, st);
-      if (e != cudaSuccess) return cuda_fail(c, e, "batch count reset");
-      a.batch_done = c->d_batch;
-    }
-    ProfScope ps(c, JNE_KERNEL_ACCUM_MIXED, st);
-    e = jne_launch_accum_mixed(a, fin, c->sms, st);
   }
+  // warps take runs from a counter, so warps that start late or finalize take fewer
+  e = cudaMemsetAsync(c->d_next_run, 0, sizeof(unsigned long long), st);
+  if (e != cudaSuccess) return cuda_fail(c, e, "work counter reset");
+  a.next_run = c->d_next_run;
+  if (fin) {
+    const size_t nb = ((size_t)n + 31) / 32;
+    int rc = ensure(c, &c->d_batch, &c->batch_cap, nb, "batch counts");
+    if (rc) return rc;
+    e = cudaMemsetAsync(c->d_batch, 0, sizeof(unsigned int) * nb, st);
+    if (e != cudaSuccess) return cuda_fail(c, e, "batch count reset");
+    a.batch_done = c->d_batch;
+  }
+  ProfScope ps(c, precision == JNE_PREC_FP64 ? JNE_KERNEL_ACCUM_FP64 : JNE_KERNEL_ACCUM_MIXED, st);
+  e = precision == JNE_PREC_FP64 ? jne_launch_accum_digits(a, fin, c->sms, st)
+                                 : jne_launch_accum_mixed(a, fin, c->sms, st);
   if (e != cudaSuccess) return cuda_fail(c, e, "accumulation launch");
   return JNE_OK;
 }
@@ -409,8 +407,7 @@ inline int check_common(jne_context* c, int model, int dim, int steps, int64_t n
 
 // Waits for the asynchronous device path, so a synchronous call owns the status word.
 inline int drain(jne_context* c) {
-  cudaError_t e = cudaStreamSynchronize(c->fin_stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaError_t e = cudaStreamSynchronize(c->stream);
   return e == cudaSuccess ? JNE_OK : cuda_fail(c, e, "drain");
 }
 
@@ -437,11 +434,10 @@ inline int join_out(jne_context* c, cudaStream_t user, int last) {
 }
 
 // Asynchronous seeded batch of one request.  Batch b uses record buffer b % 2.
-// Mixed precision: the accumulation kernel finalizes its own runs, on
-// c->stream.  FP64: the finalize of a batch runs on c->fin_stream beside the
-// next batch's accumulation.  Events order the buffer reuse; *last receives
-// the record buffer of the final batch (its ev_fin marks the results).  Device
-// status bits go to `status` (null: the context's status word).
+// The accumulation kernel finalizes its own runs, on c->stream.  Events order
+// the buffer reuse; *last receives the record buffer of the final batch (its
+// ev_fin marks the results).  Device status bits go to `status` (null: the
+// context's status word).
 inline int enqueue_seeded(jne_context* c, int model, int dim, int steps, uint64_t base_seed, uint32_t seed_first,
                           int64_t n_runs, int precision, double* out_device, int* last,
                           unsigned int* status = nullptr) {
@@ -450,7 +446,6 @@ inline int enqueue_seeded(jne_context* c, int model, int dim, int steps, uint64_
   stream_key(base_seed, dim, &k0, &k1);
   const int64_t per = batch_runs(c, dim, 0) / 2;  // two record buffers in flight
   if (per < 1) return fail(c, JNE_ERR_BUDGET, "budget too small for one run");
-  const bool fused = kernel_precision(precision, steps) == JNE_PREC_MIXED;
   cudaStream_t st = c->stream;
   cudaError_t e = cudaSuccess;
   int rc;
@@ -463,21 +458,10 @@ inline int enqueue_seeded(jne_context* c, int model, int dim, int steps, uint64_
       return rc;
     const jne_finalize_args fa =
         finalize_args(c, model, dim, steps, n, c->d_momb[b], out_device + (size_t)done * k, status);
-    if (fused) {
-      if ((rc = accumulate(c, model, dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
-                           c->d_momb[b], st, &fa, status)))
-        return rc;
-      if ((e = cudaEventRecord(c->ev_fin[b], st)) != cudaSuccess) return cuda_fail(c, e, "event record");
-    } else {
-      if ((rc = accumulate(c, model, dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
-                           c->d_momb[b], st, nullptr, status)))
-        return rc;
-      if ((e = cudaEventRecord(c->ev_acc[b], st)) != cudaSuccess ||
-          (e = cudaStreamWaitEvent(c->fin_stream, c->ev_acc[b], 0)) != cudaSuccess)
-        return cuda_fail(c, e, "stream order");
-      if ((rc = finalize(c, fa, c->fin_stream))) return rc;
-      if ((e = cudaEventRecord(c->ev_fin[b], c->fin_stream)) != cudaSuccess) return cuda_fail(c, e, "event record");
-    }
+    if ((rc = accumulate(c, model, dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
+                         c->d_momb[b], st, &fa, status)))
+      return rc;
+    if ((e = cudaEventRecord(c->ev_fin[b], st)) != cudaSuccess) return cuda_fail(c, e, "event record");
     c->fin_pending[b] = true;
     *last = b;
   }

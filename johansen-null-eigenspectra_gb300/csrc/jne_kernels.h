@@ -40,7 +40,12 @@ struct jne_ragged_req {
 cudaError_t jne_launch_accum_mixed_ragged(const jne_ragged_req* reqs, int n_req, long long total,
                                          unsigned long long* counter, unsigned int* batch_done, int sms,
                                          cudaStream_t st);
+// explicit increments (a.ext) in FP64 multiply-adds over an entry table
 cudaError_t jne_launch_accum_f64(const jne_accum_args& a, const int4* ent, int nent, int sms, cudaStream_t st);
+// The engine's own increments (a.ext == null): every Gram sum exact in digits
+// (jne_accum_digits.cuh); needs a.next_run, finalizes with fin as the mixed form.
+cudaError_t jne_launch_accum_digits(const jne_accum_args& a, const jne_finalize_args* fin, int sms, cudaStream_t st);
+cudaError_t jne_launch_accum_digits_hi(const jne_accum_args& a, const jne_finalize_args& f, int sms, cudaStream_t st);
 int jne_build_f64_entries(int model, int d, int4* out, int cap);
 // fin (may be null) finalizes the same request's runs inside the launch.
 // a.blocks_per_sm (4, or 6 for the kernels budgeted to 80 registers) and

@@ -5,15 +5,15 @@
 // that forbids foreign allocations, a real-time loop with no allocation after
 // start-up, or an embedding that only hands out device pointers for its own
 // inputs and outputs.  This entry point takes its scratch (the FP64 moment
-// records, the chunk time table, the FP64 entry table, the work and batch
-// counters and the status word) from one file-scope __device__ array of fixed
+// records, the chunk time table, the work and batch counters and the status
+// word) from one file-scope __device__ array of fixed
 // size that every GPU loading this library holds until the process exits.  It
 // calls no cudaMalloc, cudaFree or allocating library routine.
 //
 // It runs exactly the kernels and tables of the context entry point
-// (jne_eigs_seeded): the chunk table and the FP64 entry table come from the
-// same host functions, and a mixed request is the same fused accumulate +
-// finalize launch, so the two give the same bits.
+// (jne_eigs_seeded): the chunk table comes from the same host function, and a
+// request is the same fused accumulate + finalize launch, so the two give the
+// same bits.
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -26,15 +26,14 @@ namespace {
 constexpr size_t kAlign = 256;
 constexpr size_t round_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 constexpr int kRecordMax = JNE_MAX_DIM * (JNE_MAX_DIM + 1) / 2 + 6 * JNE_MAX_DIM + JNE_MAX_DIM * JNE_MAX_DIM;
-constexpr size_t kEntCap = 512;
 constexpr size_t kMomBytes = round_up(sizeof(double) * (size_t)JNE_NOALLOC_MAX_RUNS * kRecordMax);
 constexpr size_t kChunkBytes = round_up(sizeof(jne_chunk_time) * (size_t)JNE_NOALLOC_MAX_CHUNKS);
-constexpr size_t kEntBytes = round_up(sizeof(int4) * kEntCap);
+constexpr size_t kReservedBytes = 8192;  // keeps the scratch size jne.h states
 // status word (offset 0) and the mixed kernel's work counter (offset 8)
 constexpr size_t kWordsBytes = kAlign;
 // completion counts of the fused finalize, one per 32 runs
 constexpr size_t kBatchBytes = round_up(sizeof(unsigned int) * ((JNE_NOALLOC_MAX_RUNS + 31) / 32));
-constexpr size_t kScratchBytes = kMomBytes + kChunkBytes + kEntBytes + kWordsBytes + kBatchBytes;
+constexpr size_t kScratchBytes = kMomBytes + kChunkBytes + kReservedBytes + kWordsBytes + kBatchBytes;
 static_assert(kScratchBytes == JNE_NOALLOC_SCRATCH_BYTES, "scratch size stated in jne.h");
 
 static __device__ __align__(256) unsigned char jne_noalloc_scratch[kScratchBytes];
@@ -44,10 +43,9 @@ static __device__ __align__(256) unsigned char jne_noalloc_scratch[kScratchBytes
 std::mutex g_mu;
 void* g_scratch[64] = {};
 int g_sms[64] = {};
-// host staging of the tables (copied to the device under g_mu; a copy from
+// host staging of the table (copied to the device under g_mu; a copy from
 // pageable memory has read its source when the call returns)
 jne_chunk_time g_hchunk[JNE_NOALLOC_MAX_CHUNKS];
-int4 g_hent[kEntCap];
 
 thread_local std::string g_err;
 int fail(int code, const std::string& m) {
@@ -99,8 +97,7 @@ extern "C" int jne_eigs_seeded_noalloc(int device, int model, int dim, int steps
   const int sms = g_sms[device];
   double* mom = reinterpret_cast<double*>(base);
   jne_chunk_time* ctab = reinterpret_cast<jne_chunk_time*>(base + kMomBytes);
-  int4* ent = reinterpret_cast<int4*>(base + kMomBytes + kChunkBytes);
-  unsigned char* words = base + kMomBytes + kChunkBytes + kEntBytes;
+  unsigned char* words = base + kMomBytes + kChunkBytes + kReservedBytes;
   unsigned int* status = reinterpret_cast<unsigned int*>(words);
   unsigned long long* next_run = reinterpret_cast<unsigned long long*>(words + 8);
   unsigned int* batch_done = reinterpret_cast<unsigned int*>(words + kWordsBytes);
@@ -142,10 +139,9 @@ extern "C" int jne_eigs_seeded_noalloc(int device, int model, int dim, int steps
       a.batch_done = batch_done;
       if (e == cudaSuccess) e = jne_launch_accum_mixed(a, &f, sms, st);  // accumulation + fused finalize
     } else {
-      const int nent = jne_build_f64_entries(model, dim, g_hent, (int)kEntCap);
-      e = cudaMemcpyAsync(ent, g_hent, sizeof(int4) * nent, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess) e = jne_launch_accum_f64(a, ent, nent, sms, st);
-      if (e == cudaSuccess) e = jne_launch_finalize(f, sms, st);
+      a.next_run = next_run;
+      a.batch_done = batch_done;
+      e = jne_launch_accum_digits(a, &f, sms, st);
     }
   }
   lk.unlock();
