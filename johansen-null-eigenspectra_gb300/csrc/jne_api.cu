@@ -146,7 +146,7 @@ int jne_eigs_from_increments(jne_context* c, int model, int dim, int steps, cons
   if (e != cudaSuccess) return cuda_fail(c, e, "increment upload");
   jne_finalize_args fa = finalize_args(c, model, dim, steps, n_runs, c->d_mom, c->d_out);
   // FP64 walks the increments as given; the mixed kernel walks dB * sqrt(T)
-  if (kernel_precision(precision, steps) == JNE_PREC_FP64) fa.zscale = 1.0;
+  if (kernel_precision(precision, steps) == JNE_PREC_FP64) fa.lam_scale = (double)steps;
   if ((rc = accumulate(c, model, dim, steps, 0, 0, 0, n_runs, precision, c->d_ext, c->d_mom, st, &fa))) return rc;
   e = cudaMemcpyAsync(out, c->d_out, sizeof(double) * n_runs * k, cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return cuda_fail(c, e, "result download");
@@ -177,21 +177,24 @@ int jne_eigs_seeded_models(jne_context* c, const int* models, int n_models, int 
     const int n = (int)std::min<int64_t>(per, n_runs - done);
     if ((rc = ensure(c, &c->d_mom, &c->mom_cap, (size_t)n * jne_record_slots(dim), "moment buffer"))) return rc;
     if ((rc = ensure(c, &c->d_out, &c->out_cap, (size_t)n * k_total, "output buffer"))) return rc;
-    // one model: the accumulation finalizes its runs itself; several: one finalize kernel per model
+    // one model: the accumulation finalizes its runs itself; several: one finalize launch for all
     // (finalizing five models per batch inside the accumulation stalls its warps longer than the
-    // separate kernels take: 0.14 s against 0.08 s for 5 x 200k runs)
-    const jne_finalize_args f0 = finalize_args(c, models[0], dim, steps, n, c->d_mom, c->d_out);
-    if ((rc = accumulate(c, models[0], dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
-                         c->d_mom, st, n_models == 1 ? &f0 : nullptr)))
-      return rc;
+    // separate kernel takes: 0.14 s against 0.08 s for 5 x 200k runs)
+    jne_finalize_args fa[5];
     size_t off = 0;
     for (int m = 0; m < n_models; m++) {
+      fa[m] = finalize_args(c, models[m], dim, steps, n, c->d_mom, c->d_out + off);
+      off += (size_t)n * jne_eigen_count(models[m], dim);
+    }
+    if ((rc = accumulate(c, models[0], dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
+                         c->d_mom, st, n_models == 1 ? fa : nullptr)))
+      return rc;
+    if (n_models > 1 && (rc = finalize(c, fa, n_models, st))) return rc;
+    for (int m = 0; m < n_models; m++) {
       const int k = jne_eigen_count(models[m], dim);
-      if (n_models > 1 && (rc = finalize(c, models[m], dim, steps, n, c->d_mom, c->d_out + off, st))) return rc;
-      cudaError_t e = cudaMemcpyAsync(outs[m] + (size_t)done * k, c->d_out + off, sizeof(double) * n * k,
+      cudaError_t e = cudaMemcpyAsync(outs[m] + (size_t)done * k, fa[m].out, sizeof(double) * n * k,
                                       cudaMemcpyDeviceToHost, st);
       if (e != cudaSuccess) return cuda_fail(c, e, "result download");
-      off += (size_t)n * k;
     }
   }
   return check_status(c);

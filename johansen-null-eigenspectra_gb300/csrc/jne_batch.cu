@@ -68,7 +68,7 @@ void describe(jne_context* c, const jne_request* reqs, double* const* outs, cons
     d.fin.dim = r.dim;
     d.fin.steps = r.steps;
     d.fin.n_runs = (int)p.n;
-    d.fin.zscale = 1.0 / std::sqrt((double)r.steps);
+    d.fin.lam_scale = 1.0;
     d.fin.ts = time_sums(r.steps);
     d.fin.mom = mom + moff;
     d.fin.mom_ld = p.n;

@@ -125,7 +125,7 @@ __device__ __forceinline__ void jne_normal_quad(uint32_t s, uint32_t j, uint32_t
 
 // ---------------------------------------------------------------------------
 // Per-run moment record (FP64), in units of the unscaled walk W_i = sum_{s<=i} z_s
-// (B = zscale * W, dB = zscale * z).  Column i = 0..T-1 pairs W_i (B_{t-1})
+// (B = W / sqrt(T), dB = z / sqrt(T); explicit increments in FP64: B = W).  Column i = 0..T-1 pairs W_i (B_{t-1})
 // with the increment z_{i+1} and the time point y_i = (i+1)/T.
 //   [0, d(d+1)/2)        MWW[a][b] = sum W_a W_b        (a <= b, row-major upper)
 //   +d                   MW1[a]    = sum W_a

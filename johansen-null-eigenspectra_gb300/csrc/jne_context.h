@@ -230,6 +230,12 @@ inline jne_time_sums time_sums(int steps) {
   s.Y[2] = (double)((T + 1.0L) * (2.0L * T + 1.0L) / (6.0L * T));
   s.Y[3] = (double)((T + 1.0L) * (T + 1.0L) / (4.0L * T));
   s.Y[4] = (double)((T + 1.0L) * (2.0L * T + 1.0L) * (3.0L * T * T + 3.0L * T - 1.0L) / (30.0L * T * T * T));
+  // centred: sum (y - ybar)^2 = (T^2 - 1) / (12 T), sum (y - ybar) y^2 = (T + 1)(T^2 - 1) / (12 T^2),
+  // sum (y - 1/2)^2 = (T^2 + 2) / (12 T), and the residual of y^2 on {1, y}: (T^2 - 1)(T^2 - 4) / (180 T^3)
+  s.Syy = (double)((T * T - 1.0L) / (12.0L * T));
+  s.Syy2 = (double)((T + 1.0L) * (T * T - 1.0L) / (12.0L * T * T));
+  s.Syh = (double)((T * T + 2.0L) / (12.0L * T));
+  s.Sr2 = (double)((T * T - 1.0L) * (T * T - 4.0L) / (180.0L * T * T * T));
   return s;
 }
 
@@ -283,7 +289,7 @@ inline int kernel_precision(int precision, int steps) {
   return (precision == JNE_PREC_MIXED && steps >= JNE_MIXED_MIN_STEPS) ? JNE_PREC_MIXED : JNE_PREC_FP64;
 }
 
-inline int finalize(jne_context* c, const jne_finalize_args& f, cudaStream_t st);
+inline int finalize(jne_context* c, const jne_finalize_args* f, int n, cudaStream_t st);
 
 // The finalize argument block of n runs of one request (records in mom);
 // device status bits go to `status` (null: the context's status word).
@@ -294,7 +300,7 @@ inline jne_finalize_args finalize_args(jne_context* c, int model, int dim, int s
   f.dim = dim;
   f.steps = steps;
   f.n_runs = n;
-  f.zscale = 1.0 / std::sqrt((double)steps);
+  f.lam_scale = 1.0;
   f.ts = time_sums(steps);
   f.mom = mom;
   f.mom_ld = n;
@@ -343,7 +349,7 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
       e = jne_launch_accum_f64(a, c->d_ent, c->ent_n, c->sms, st);
     }
     if (e != cudaSuccess) return cuda_fail(c, e, "accumulation launch");
-    return fin ? finalize(c, *fin, st) : JNE_OK;
+    return fin ? finalize(c, fin, 1, st) : JNE_OK;
   }
   if (precision == JNE_PREC_MIXED) {
     // per-chunk time means, exact (integer sums) then rounded once
@@ -382,16 +388,11 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
   return JNE_OK;
 }
 
-inline int finalize(jne_context* c, const jne_finalize_args& f, cudaStream_t st) {
+inline int finalize(jne_context* c, const jne_finalize_args* f, int n, cudaStream_t st) {
   ProfScope ps(c, JNE_KERNEL_FINALIZE, st);
-  cudaError_t e = jne_launch_finalize(f, c->sms, st);
+  cudaError_t e = jne_launch_finalize(f, n, st);
   if (e != cudaSuccess) return cuda_fail(c, e, "finalize launch");
   return JNE_OK;
-}
-
-inline int finalize(jne_context* c, int model, int dim, int steps, int n, const double* mom, double* d_out,
-                    cudaStream_t st) {
-  return finalize(c, finalize_args(c, model, dim, steps, n, mom, d_out), st);
 }
 
 inline int check_common(jne_context* c, int model, int dim, int steps, int64_t n_runs, int precision) {

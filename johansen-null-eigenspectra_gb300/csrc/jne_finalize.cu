@@ -1,26 +1,34 @@
-// jne_finalize.cu -- the finalize kernels: one thread per run turns the run's
+// jne_finalize.cu -- the finalize kernel: one thread per run turns the run's
 // moment record into its eigenvalues (jne_finalize_run.cuh; replaces
-// johansen_statistics.rs:24-47).  Used by the FP64 path and by multi-model
-// requests (one accumulation, one finalize per model); the mixed kernels
-// finalize their own runs.
+// johansen_statistics.rs:24-47).  Used by multi-model requests (one accumulation,
+// then every model of every run in one launch) and by explicit increments in
+// FP64; the other kernels finalize their own runs.
 #include "jne_finalize_run.cuh"
 
 namespace {
 
+// Blocks of two warps: few enough for the last wave to fill, and all models in
+// one grid, so that only the launch's own tail leaves SMs idle.
 constexpr int kFinThreads = 64;
-using jne_fin::finalize_run;
 
-__global__ void __launch_bounds__(kFinThreads) k_finalize(const jne_finalize_args f) {
+struct FinalizeList {
+  jne_finalize_args f[5];
+};
+
+__global__ void __launch_bounds__(kFinThreads) k_finalize(const __grid_constant__ FinalizeList list) {
+  const jne_finalize_args& f = list.f[blockIdx.y];
   const int run = blockIdx.x * kFinThreads + threadIdx.x;
-  if (run < f.n_runs) finalize_run(f, run);
+  if (run < f.n_runs) jne_fin::finalize_run(f, run);
 }
 
 }  // namespace
 
-cudaError_t jne_launch_finalize(const jne_finalize_args& f, int sms, cudaStream_t st) {
-  (void)sms;
-  if (f.n_runs <= 0) return cudaSuccess;
-  const int grid = (f.n_runs + kFinThreads - 1) / kFinThreads;
-  k_finalize<<<grid, kFinThreads, 0, st>>>(f);
+cudaError_t jne_launch_finalize(const jne_finalize_args* f, int n, cudaStream_t st) {
+  if (n < 1 || n > 5) return cudaErrorInvalidValue;
+  if (f[0].n_runs <= 0) return cudaSuccess;
+  FinalizeList list{};
+  for (int i = 0; i < n; i++) list.f[i] = f[i];
+  const dim3 grid((f[0].n_runs + kFinThreads - 1) / kFinThreads, n);
+  k_finalize<<<grid, kFinThreads, 0, st>>>(list);
   return cudaGetLastError();
 }

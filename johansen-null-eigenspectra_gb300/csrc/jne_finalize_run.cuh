@@ -5,17 +5,31 @@
 // Replaces johansen_statistics.rs:24-47 (the F-based Grams, then
 // GeneralizedEigen(S10'S10, S11) via LAPACK dggev, |alpha|/beta, descending
 // sort).  One thread per run, all in FP64:
-//   1. F_j = G[x_j] - alpha_j * 1 - beta_j * y for the model's rows, where
-//      G = [B; 1; y; y^2].  This is construct_f_matrix (:102-197) written as a
-//      linear map: demeaning (models 2, 3) subtracts the row mean, model 4
-//      subtracts the least-squares fit on {1, y}.  S11 = dt F F' and
-//      S10 = dB F' then follow from the raw moments alone.
-//   2. S11 = L L' (Cholesky), E = S10 L^-T, C = E'E: the pencil's eigenvalues
-//      are those of the symmetric PSD matrix C.
-//   3. Householder tridiagonalisation + implicit QL (eigenvalues only), then
-//      |lambda| and a descending sort -- the reference reports |alpha|/beta.
-// The QL path needs ~10x fewer FP64 operations than cyclic Jacobi at k = 13,
-// which matters on a GPU whose FP64 rate is ~1/74 of its FP32 rate.
+//   1. F_j = G[x_j] - alpha_j * 1 - beta_j * (y - ybar) for the model's rows,
+//      where G = [W; 1; y; y^2].  This is construct_f_matrix (:102-197) written as
+//      a linear map: demeaning (models 2, 3) subtracts the row mean, model 4
+//      subtracts the least-squares fit on {1, y}, here on the orthogonal pair
+//      {1, y - ybar}.  A residual is orthogonal to what was subtracted, so
+//      F_j F_l' = F_j G_l' needs one side's correction.
+//      The walk stays unscaled: scaling a row of F does not change the pencil's
+//      eigenvalues, and the factors dt of S11 and s^2 of S10'S10 (dB = s z) are
+//      one factor of the result (lam_scale).
+//   2. S11 = L L' (Cholesky, reciprocal pivots only), E = S10 L^-T, C = E'E: the
+//      pencil's eigenvalues are those of the symmetric PSD matrix C.
+//   3. Householder tridiagonalisation of one triangle + implicit QL (eigenvalues
+//      only), then |lambda| and a descending sort -- the reference reports
+//      |alpha|/beta.
+// What bounds it: FP64 instructions.  On this GPU one warp's FP64 instruction
+// holds its scheduler's FP64 pipe for 64 cycles (76 with all four busy), however
+// many of its lanes are active, and dependent ones follow each other as fast as
+// independent ones; so a warp finalizes 32 runs, one per lane, and the time is the
+// instruction count.  At k = 13 about 7,500 are left of 12,000: the one-sided
+// corrections and the unscaled walk (S, S10), rsqrt for sqrt and division, half the
+// rank-two updates, the shift's correction in FP32 (any shift is a valid one: only
+// the convergence depends on it) and the deflation test on exponents.
+// Measured: five models of 40,000 runs at dim 12, T 2000 (one launch for all models
+// included) 11.25 -> 7.70 ms; 20,011 runs at dim 6, T 100, mostly finalize, 563 -> 447 us;
+// errors against quad precision no larger (dim 12, T 100, model 4: 4.1e-14 -> 2.3e-14 rms).
 #pragma once
 #include <cfloat>
 #include <math_constants.h>
@@ -24,64 +38,88 @@
 namespace jne_fin {
 namespace {  // internal linkage: each translation unit that includes this has its own copy
 
+// The run's moment record, in units of the unscaled walk.
 struct Ctx {
   const double* mom;
   long long ld;
   int run, d;
-  double s;
   const double* Y;
   // cached in L2 only: the mixed kernel reads records its own warp wrote moments earlier
   __device__ double rec(int slot) const { return __ldcg(mom + (size_t)slot * ld + run); }
-  // M(r, n) = sum_i G_r G_n over the global basis G = [B (d); 1; y; y^2]
+  // M(r, n) = sum_i G_r G_n over the global basis G = [W (d); 1; y; y^2], r <= n
   __device__ double M(int r, int n) const {
-    if (r > n) { const int t = r; r = n; n = t; }
-    if (n < d) return s * s * rec(jne_slot_MWW(r, n, d));
+    if (n < d) return rec(jne_slot_MWW(r, n, d));
     if (r < d) {
       const int p = n - d;
-      return s * rec(p == 0 ? jne_slot_MW1(r, d) : p == 1 ? jne_slot_MWy(r, d) : jne_slot_MWyy(r, d));
+      return rec(p == 0 ? jne_slot_MW1(r, d) : p == 1 ? jne_slot_MWy(r, d) : jne_slot_MWyy(r, d));
     }
     return Y[(r - d) + (n - d)];
   }
-  // N(r, c) = sum_i G_r dB_c
+  // N(r, c) = sum_i G_r z_c
   __device__ double N(int r, int c) const {
-    if (r < d) return s * s * rec(jne_slot_NzW(c, r, d));
+    if (r < d) return rec(jne_slot_NzW(c, r, d));
     const int p = r - d;
-    return s * rec(p == 0 ? jne_slot_Nz1(c, d) : p == 1 ? jne_slot_Nzy(c, d) : jne_slot_Nzyy(c, d));
+    return rec(p == 0 ? jne_slot_Nz1(c, d) : p == 1 ? jne_slot_Nzy(c, d) : jne_slot_Nzyy(c, d));
   }
 };
 
-// Householder reduction of the symmetric n x n matrix A (full storage) to
-// tridiagonal form (Golub & Van Loan, Matrix Computations, Algorithm 8.3.1):
-// diagonal -> dg[0..n-1], sub-diagonal -> eo[0..n-2].
+// 1 / x for normal x: the documented approximation and one third-order Newton
+// step (Householder's method), three FP64 instructions.
+__device__ __forceinline__ double reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// Householder reduction of a symmetric n x n matrix to tridiagonal form (Golub &
+// Van Loan, Matrix Computations, Algorithm 8.3.1), given and overwritten as its
+// strict upper triangle (A[i][j], i < j) and diagonal: diagonal -> dg[0..n-1],
+// sub-diagonal -> eo[0..n-2].
 __device__ __forceinline__ void tridiagonalize(double (*A)[JNE_MAX_K], int n, double* dg, double* eo) {
   for (int k = 0; k + 2 < n; k++) {
     double sigma = 0.0;
-    for (int i = k + 2; i < n; i++) sigma += A[i][k] * A[i][k];
-    const double x0 = A[k + 1][k];
+    for (int i = k + 2; i < n; i++) sigma = fma(A[k][i], A[k][i], sigma);
+    const double x0 = A[k][k + 1];
     if (sigma == 0.0) { eo[k] = x0; continue; }
-    const double nrm = sqrt(x0 * x0 + sigma);
+    const double r2 = fma(x0, x0, sigma);
+    const double nrm = r2 * rsqrt(r2);
     const double alpha = x0 > 0.0 ? -nrm : nrm;  // H x = alpha e1
-    double v[JNE_MAX_K];
+    double v[JNE_MAX_K], p[JNE_MAX_K];
     v[k + 1] = x0 - alpha;                        // |x0| + nrm: no cancellation
-    for (int i = k + 2; i < n; i++) v[i] = A[i][k];
-    const double tau = 1.0 / (nrm * (nrm + fabs(x0)));  // 2 / (v'v)
-    double p[JNE_MAX_K];
+    for (int i = k + 2; i < n; i++) v[i] = A[k][i];
+    const double tau = reciprocal(fma(nrm, fabs(x0), r2));  // 2 / (v'v)
+    for (int i = k + 1; i < n; i++) p[i] = dg[i] * v[i];
+    for (int i = k + 1; i < n; i++) {
+      const double vi = v[i];
+      double t = p[i];
+      for (int j = i + 1; j < n; j++) {
+        const double a = A[i][j];
+        t = fma(a, v[j], t);
+        p[j] = fma(a, vi, p[j]);
+      }
+      p[i] = t;
+    }
     double pv = 0.0;
     for (int i = k + 1; i < n; i++) {
-      double t = 0.0;
-      for (int j = k + 1; j < n; j++) t += A[i][j] * v[j];
-      p[i] = tau * t;
-      pv += p[i] * v[i];
+      p[i] *= tau;
+      pv = fma(p[i], v[i], pv);
     }
     const double K = 0.5 * tau * pv;
-    for (int i = k + 1; i < n; i++) p[i] -= K * v[i];  // w = p - K v
-    for (int i = k + 1; i < n; i++)
-      for (int j = k + 1; j < n; j++) A[i][j] -= v[i] * p[j] + p[i] * v[j];
+    for (int i = k + 1; i < n; i++) p[i] = fma(-K, v[i], p[i]);  // w = p - K v
+    for (int i = k + 1; i < n; i++) {
+      const double vi = v[i], wi = p[i];
+      dg[i] = fma(-2.0 * vi, wi, dg[i]);
+      for (int j = i + 1; j < n; j++) A[i][j] = fma(-wi, v[j], fma(-vi, p[j], A[i][j]));
+    }
     eo[k] = alpha;
   }
-  if (n >= 2) eo[n - 2] = A[n - 1][n - 2];
-  for (int i = 0; i < n; i++) dg[i] = A[i][i];
+  if (n >= 2) eo[n - 2] = A[n - 2][n - 1];
 }
+
+// Biased exponent field of a double, as an integer to compare.
+__device__ __forceinline__ int exponent_bits(double x) { return __double2hiint(x) & 0x7FF00000; }
+__device__ __forceinline__ bool is_zero(double x) { return ((__double2hiint(x) & 0x7FFFFFFF) | __double2loint(x)) == 0; }
 
 // Eigenvalues of the symmetric tridiagonal matrix (dg, eo) by the implicit QL
 // method with Wilkinson shifts (Bowdler, Martin, Reinsch & Wilkinson, "The QR
@@ -93,15 +131,24 @@ __device__ __forceinline__ bool tridiagonal_ql(double* dg, double* eo, int n) {
   for (int l = 0; l < n; l++) {
     for (int iter = 0; iter < 64; iter++) {
       int m = l;
+      // negligible by exponents, with no FP64 instruction: |eo| < eps max(|dg[m]|, |dg[m + 1]|) when it
+      // breaks, within a factor of four of |eo| <= eps (|dg[m]| + |dg[m + 1]|); never for a NaN
+      int em = exponent_bits(dg[l]);
       for (; m < n - 1; m++) {
-        const double dd = fabs(dg[m]) + fabs(dg[m + 1]);
-        if (fabs(eo[m]) <= DBL_EPSILON * dd) break;
+        const int en = exponent_bits(dg[m + 1]);
+        if (exponent_bits(eo[m]) <= max(em, en) - (53 << 20) || is_zero(eo[m])) break;
+        em = en;
       }
       if (m == l) break;
       if (iter == 63) { ok = false; break; }
-      double g = (dg[l + 1] - dg[l]) / (2.0 * eo[l]);
-      double r = hypot(g, 1.0);
-      g = dg[m] - dg[l] + eo[l] / (g + copysign(r, g));
+      // the shift d_l - e_l / (g + sign(g) sqrt(g^2 + 1)), g = (d_{l+1} - d_l) / (2 e_l): its correction in FP32
+      const float ef = (float)eo[l], gf = (float)(dg[l + 1] - dg[l]) / (2.0f * ef);
+      double cf = (double)(ef / (gf + copysignf(sqrtf(fmaf(gf, gf, 1.0f)), gf)));
+      if (!isfinite(cf)) {  // values outside FP32's range
+        const double gd = (dg[l + 1] - dg[l]) / (2.0 * eo[l]);
+        cf = eo[l] / (gd + copysign(hypot(gd, 1.0), gd));
+      }
+      double g = dg[m] - dg[l] + cf;
       double s = 1.0, c = 1.0, p = 0.0;
       int i = m - 1;
       bool underflow = false;
@@ -118,15 +165,14 @@ __device__ __forceinline__ bool tridiagonal_ql(double* dg, double* eo, int n) {
           break;
         }
         const double ir = rsqrt(r2);
-        r = r2 * ir;
-        eo[i + 1] = r;
+        eo[i + 1] = r2 * ir;
         s = f * ir;
         c = g * ir;
         g = dg[i + 1] - p;
-        r = (dg[i] - g) * s + 2.0 * c * b;
+        const double r = fma(dg[i] - g, s, 2.0 * c * b);
         p = s * r;
         dg[i + 1] = g + p;
-        g = c * r - b;
+        g = fma(c, r, -b);
       }
       if (underflow) continue;
       dg[l] -= p;
@@ -140,53 +186,55 @@ __device__ __forceinline__ bool tridiagonal_ql(double* dg, double* eo, int n) {
 __device__ __noinline__ void finalize_run(const jne_finalize_args& f, int run) {
   const int d = f.dim, model = f.model;
   const int k = (model == 1 || model == 3) ? d + 1 : d;
-  const Ctx c{f.mom, f.mom_ld, run, d, f.zscale, f.ts.Y};
-  const double T = (double)f.steps, dt = 1.0 / T;
-  const double Y0 = f.ts.Y[0], Y1 = f.ts.Y[1], Y2 = f.ts.Y[2];
+  const Ctx c{f.mom, f.mom_ld, run, d, f.ts.Y};
+  const double T = (double)f.steps;
   const int ONE = d, Yr = d + 1, YY = d + 2;
+  const int nb = (model == 2 || model == 4) ? d - 1 : d;    // walk rows kept
+  const int last = model == 1 ? ONE : model == 4 ? YY : Yr;  // the row after them (none in model 0)
+  const bool trend = model == 2 || model == 3;              // its row is y - 1/2
+  const int proj = trend ? 1 : model == 4 ? 2 : 0;          // corrections: 1, or 1 and y
 
-  // F rows: F_j = G[x_j] - al_j * G[ONE] - be_j * G[Yr]
-  int x[JNE_MAX_K];
+  // F rows: F_j = G[x_j] - al_j * 1 - be_j * (y - ybar)
   double al[JNE_MAX_K], be[JNE_MAX_K], m1[JNE_MAX_K], my[JNE_MAX_K];
-  const int nb = (model == 2 || model == 4) ? d - 1 : d;  // walk rows kept
-  for (int j = 0; j < k; j++) {
-    x[j] = j < nb ? j : (model == 1 ? ONE : model == 4 ? YY : Yr);
-    m1[j] = c.M(x[j], ONE);
-    my[j] = c.M(x[j], Yr);
-    al[j] = 0.0;
-    be[j] = 0.0;
-  }
-  if (model == 2 || model == 3) {
-    for (int j = 0; j < nb; j++) al[j] = m1[j] / T;  // row mean
-    al[nb] = 0.5;                                    // trend row y - 0.5
-  } else if (model == 4) {
-    const double det = Y0 * Y2 - Y1 * Y1;
-    const double i00 = Y2 / det, i01 = -Y1 / det, i11 = Y0 / det;
+  const double iT = 1.0 / T, ybar = f.ts.Y[1] * iT;
+  if (proj >= 1)
+    for (int j = 0; j < nb; j++) {
+      m1[j] = c.M(j, ONE);
+      al[j] = m1[j] * iT;  // row mean
+    }
+  if (trend) al[nb] = 0.5;
+  if (proj == 2) {
+    const double iS = 1.0 / f.ts.Syy;
+    m1[nb] = f.ts.Y[2];
+    al[nb] = m1[nb] * iT;
     for (int j = 0; j < k; j++) {
-      al[j] = m1[j] * i00 + my[j] * i01;
-      be[j] = m1[j] * i01 + my[j] * i11;
+      my[j] = j < nb ? fma(-ybar, m1[j], c.M(j, Yr)) : f.ts.Syy2;  // sum (y - ybar) G_j
+      be[j] = my[j] * iS;
     }
   }
 
+  // S11 (lower triangle of S) and its Cholesky factor, row by row; inv[j] = 1 / L[j][j]
   double S[JNE_MAX_K][JNE_MAX_K];
-  for (int j = 0; j < k; j++)
-    for (int l = 0; l <= j; l++) {
-      double v = c.M(x[j], x[l]) - al[l] * m1[j] - be[l] * my[j] - al[j] * m1[l] - be[j] * my[l] +
-                 al[j] * al[l] * Y0 + (al[j] * be[l] + be[j] * al[l]) * Y1 + be[j] * be[l] * Y2;
-      S[j][l] = v * dt;
-    }
-
-  // Cholesky S11 = L L' (lower triangle of S); inv[j] = 1 / L[j][j]
   bool ok = true;
   double inv[JNE_MAX_K];
   for (int j = 0; j < k && ok; j++) {
+    const int x = j < nb ? j : last;
     for (int i = 0; i <= j; i++) {
-      double s = S[j][i];
-      for (int p = 0; p < i; p++) s -= S[j][p] * S[i][p];
+      double s;
+      if (trend && j == nb) {
+        // (y - 1/2) against the demeaned walk i (sum (y - 1/2) = 1/2), and against itself
+        s = i < nb ? fma(-0.5, m1[i] + al[i], c.M(i, Yr)) : f.ts.Syh;
+      } else if (proj == 2 && i == nb) {
+        s = f.ts.Sr2;  // the residual of y^2
+      } else {
+        s = i < nb ? c.M(i, x) : c.M(x, x);
+        if (proj >= 1) s = fma(-al[j], m1[i], s);
+        if (proj == 2) s = fma(-be[j], my[i], s);
+      }
+      for (int p = 0; p < i; p++) s = fma(-S[j][p], S[i][p], s);
       if (i == j) {
         if (!(s > 0.0)) { ok = false; break; }
-        S[j][j] = sqrt(s);
-        inv[j] = 1.0 / S[j][j];
+        inv[j] = rsqrt(s);
       } else {
         S[j][i] = s * inv[i];
       }
@@ -201,34 +249,30 @@ __device__ __noinline__ void finalize_run(const jne_finalize_args& f, int run) {
   // C = E'E with E = S10 L^-T, one row of E at a time: row cc solves
   // L e = S10[cc, :]' and adds e e' to C, so E is never stored.  C's strict
   // upper triangle lives in the upper triangle of S (L uses the lower one and
-  // inv[] its diagonal), its diagonal in cd[].
-  double cd[JNE_MAX_K];
+  // inv[] its diagonal), its diagonal in dg[].
+  double dg[JNE_MAX_K], eo[JNE_MAX_K];
   for (int p = 0; p < k; p++) {
-    cd[p] = 0.0;
+    dg[p] = 0.0;
     for (int q = p + 1; q < k; q++) S[p][q] = 0.0;
   }
   for (int cc = 0; cc < d; cc++) {
-    const double n1 = c.N(ONE, cc), ny = c.N(Yr, cc);
+    const double n1 = proj >= 1 ? c.N(ONE, cc) : 0.0, ny = proj == 2 ? fma(-ybar, n1, c.N(Yr, cc)) : 0.0;
     double e[JNE_MAX_K];
     for (int j = 0; j < k; j++) {
-      double s = c.N(x[j], cc) - al[j] * n1 - be[j] * ny;
-      for (int p = 0; p < j; p++) s -= S[j][p] * e[p];
+      double s = c.N(j < nb ? j : last, cc);
+      if (proj >= 1) s = fma(-al[j], n1, s);
+      if (proj == 2) s = fma(-be[j], ny, s);
+      for (int p = 0; p < j; p++) s = fma(-S[j][p], e[p], s);
       e[j] = s * inv[j];
     }
     for (int p = 0; p < k; p++) {
-      cd[p] += e[p] * e[p];
-      for (int q = 0; q < p; q++) S[q][p] += e[p] * e[q];
+      dg[p] = fma(e[p], e[p], dg[p]);
+      for (int q = 0; q < p; q++) S[q][p] = fma(e[p], e[q], S[q][p]);
     }
   }
-  // full symmetric storage for the tridiagonalisation
-  for (int p = 0; p < k; p++) {
-    S[p][p] = cd[p];
-    for (int q = 0; q < p; q++) S[p][q] = S[q][p];
-  }
-  double dg[JNE_MAX_K], eo[JNE_MAX_K];
   tridiagonalize(S, k, dg, eo);
   if (!tridiagonal_ql(dg, eo, k) && f.status) atomicOr(f.status, JNE_DEV_NOT_SPD);
-  for (int j = 0; j < k; j++) dg[j] = fabs(dg[j]);
+  for (int j = 0; j < k; j++) dg[j] = fabs(dg[j]) * f.lam_scale;
   for (int j = 1; j < k; j++) {  // insertion sort, descending
     const double v = dg[j];
     int i = j - 1;

@@ -3,9 +3,12 @@
 #include <cuda_runtime.h>
 #include "jne_common.cuh"
 
-// Deterministic time sums Y[p] = sum_{i=0}^{T-1} ((i+1)/T)^p, p = 0..4.
+// Deterministic time sums over y = (i+1)/T, i = 0..T-1: Y[p] = sum y^p, p = 0..4;
+// Syy = sum (y - ybar)^2, Syy2 = sum (y - ybar) y^2, Syh = sum (y - 1/2)^2, and
+// Sr2, the sum of squares of y^2 less its fit on {1, y}.
 struct jne_time_sums {
   double Y[5];
+  double Syy, Syy2, Syh, Sr2;
 };
 
 // The mixed kernels can pack two runs into one warp ("unit") for dims up to
@@ -18,7 +21,7 @@ __host__ __device__ __forceinline__ long long jne_units(int dim, long long n_run
 // Argument block of the finalize kernel.
 struct jne_finalize_args {
   int model, dim, steps, n_runs;
-  double zscale;            // B = zscale * W, dB = zscale * z
+  double lam_scale;         // eigenvalues = lam_scale x those of the records' pencil (s^2 T for B = s W)
   jne_time_sums ts;
   const double* mom;        // moment records (SoA)
   long long mom_ld;
@@ -55,7 +58,8 @@ cudaError_t jne_launch_accum_mixed(const jne_accum_args& a, const jne_finalize_a
 cudaError_t jne_launch_accum_mixed_b6(const jne_accum_args& a, const jne_finalize_args* fin, int sms, cudaStream_t st);
 cudaError_t jne_launch_accum_mixed_ext(const jne_accum_args& a, const jne_finalize_args* fin, int sms,
                                        cudaStream_t st);
-cudaError_t jne_launch_finalize(const jne_finalize_args& f, int sms, cudaStream_t st);
+// n (1..5) finalizes over the same number of runs in one launch
+cudaError_t jne_launch_finalize(const jne_finalize_args* f, int n, cudaStream_t st);
 // The .dat records of n results of consecutive seeds (jne_pack.cu): out is
 // 16-byte aligned and holds jne_records_bytes(seed_first, n, k) bytes.
 cudaError_t jne_launch_pack_records(const double* eigs, unsigned char* out, uint32_t seed_first, long long n, int k,

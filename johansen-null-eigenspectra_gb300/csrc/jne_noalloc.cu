@@ -122,7 +122,7 @@ extern "C" int jne_eigs_seeded_noalloc(int device, int model, int dim, int steps
   f.dim = dim;
   f.steps = steps;
   f.n_runs = n_runs;
-  f.zscale = 1.0 / std::sqrt((double)steps);
+  f.lam_scale = 1.0;
   f.ts = time_sums(steps);
   f.mom = mom;
   f.mom_ld = n_runs;
