@@ -4,12 +4,21 @@
 // Max aggregate of every run's eigenvalues (:26-39), then the percentiles with
 // the interpolation rule of get_percentile_value (:4-18).  The reference sorts
 // all aggregates; only the two order statistics around each rank p (n - 1) are
-// needed, so they are found by a most-significant-digit radix select on
-// order-preserving 64-bit keys: 8 passes of 8 bits over the n keys, each pass
-// one histogram per wanted rank (restricted to the keys that share the rank's
-// prefix found so far).  The selected keys are exact aggregate values, and the
-// interpolation runs on the host with the reference's arithmetic, so the
-// result is bit-identical to a full sort.
+// needed, so they are found by a most-significant-digit select on
+// order-preserving 64-bit keys less their minimum: a first histogram of up to
+// 2048 bins over the keys' actual range, then 7 bits a pass for each wanted rank's
+// bin, until a bin holds at most 64 keys, which the next pass lists.  The selected
+// keys are exact aggregate values, and the interpolation runs on the host with the
+// reference's arithmetic, so the result is bit-identical to a full sort.
+//
+// What bounds it: for 10^6 runs of 12 values the 96 MB read (15 us at the copy
+// bandwidth) and, for the sums, the FP64 additions (19 us); the passes read 8 MB of
+// keys from L2, and all but the first skip a key by one bit of a map of the selected
+// first bins.  Each pass's last block picks the bins and clears the counters, so a
+// pass is one launch; three resolve distinct values, and the host starts more only
+// when they did not.  10^6 x 12, seven percentiles: 444 us before (eight passes of
+// three launches, each comparing every key with every rank's prefix), 130 now, of
+// which 69 are what a call of 100 rows takes (four launches, a copy and the waits).
 #include <cfloat>
 #include <cstring>
 #include "jne_context.h"
@@ -19,7 +28,11 @@ using namespace jne_detail;
 namespace {
 
 constexpr int kQThreads = 256;
-constexpr int kGroup = 16;  // ranks per select group (16 x 256 histogram bins in shared memory)
+constexpr int kPassThreads = 512;
+constexpr int kGroup = 16;      // ranks per select group
+constexpr int kFirstMax = 2048;  // bins of the first pass
+constexpr int kSubBits = 7, kSub = 1 << kSubBits;
+constexpr int kList = kSub / 2;  // keys that fit a rank's counters
 
 // Order-preserving map of doubles to unsigned keys: negative values flip all
 // bits, non-negative values set the sign bit.
@@ -35,69 +48,281 @@ double value_of(unsigned long long k) {
   return v;
 }
 
+// Select state in device memory, ahead of the per-rank arrays.
+struct QHead {
+  unsigned int n_nan, ticket;
+  unsigned long long neg_min, max;  // ~smallest and largest key (both start at 0)
+  unsigned long long todo;          // ranks of the group still open (bit per rank)
+};
+constexpr int kHeadWords = sizeof(QHead) / 8 + 1;  // and the shifts
+
+// The scratch after the keys.
+struct QLayout {
+  QHead* head;
+  unsigned int* shifts;        // [0] bits below the first digit, [1] below the current one
+  unsigned long long* prefix;  // per rank: (key - min) >> shifts[1]; the key itself once closed
+  unsigned long long* rank;    // per rank: rank within its bin
+  unsigned long long* count;   // per rank: keys in its bin, twice (high and low half)
+  unsigned int* map;           // first-pass bins selected by some rank (a bit each)
+  unsigned int* hist;          // bins of the current pass (kSub per rank after the first), or a small bin's keys
+};
+
+struct QRanks {
+  unsigned long long r[kGroup];
+};
+
+// First-pass bins for a group of nr ranks: what keeps the scratch within 256
+// counters a rank.
+int first_bins(int nr) {
+  int b = kSub;
+  while (2 * b <= 256 * nr - 64 && 2 * b <= kFirstMax) b *= 2;
+  return b;
+}
+
 // Sum (in index order, as the reference's iterator sum) or max (folded from
-// f64::MIN) of each run's k eigenvalues; counts NaN aggregates.
-__global__ void k_aggregate(const double* __restrict__ eigs, long long n, int k, int stat,
-                            unsigned long long* __restrict__ keys, unsigned int* __restrict__ n_nan) {
+// f64::MIN, NaN ignored) of each run's k eigenvalues, as keys, with their
+// smallest and largest; counts NaN aggregates.
+// Values of a row are loaded eight at a time ahead of their (sequential) use.
+template <bool PAIRS>
+__global__ void __launch_bounds__(kQThreads) k_aggregate(const double* __restrict__ eigs, long long n, int k, int stat,
+                                                         unsigned long long* __restrict__ keys, QHead* head) {
   const long long stride = (long long)gridDim.x * blockDim.x;
+  unsigned long long lo = ~0ull, hi = 0ull;
   for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
     const double* e = eigs + r * k;
-    double a = stat == 0 ? 0.0 : -DBL_MAX;
-    for (int j = 0; j < k; j++) a = stat == 0 ? __dadd_rn(a, e[j]) : fmax(a, e[j]);
-    if (a != a) atomicAdd(n_nan, 1u);
-    keys[r] = key_of(a);
+    unsigned long long key = key_of(-DBL_MAX);
+    double a = 0.0;
+    for (int j0 = 0; j0 < k; j0 += 8) {
+      double v[8];
+      if (PAIRS) {
+#pragma unroll
+        for (int j = 0; j < 8; j += 2)
+          if (j0 + j < k) {
+            const double2 p = *reinterpret_cast<const double2*>(e + j0 + j);
+            v[j] = p.x;
+            v[j + 1] = p.y;
+          }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (j0 + j < k) v[j] = e[j0 + j];
+      }
+      if (stat == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (j0 + j < k) a = __dadd_rn(a, v[j]);
+      } else {  // max on the keys, without FP64 instructions (beyond the infinities' keys lie NaNs)
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (j0 + j < k) {
+            const unsigned long long c = key_of(v[j]);
+            if (c > key && c <= 0xFFF0000000000000ull) key = c;
+          }
+      }
+    }
+    if (stat == 0) {
+      if (a != a) atomicAdd(&head->n_nan, 1u);
+      key = key_of(a);
+    }
+    keys[r] = key;
+    lo = min(lo, key);
+    hi = max(hi, key);
+  }
+  for (int o = 16; o; o >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  __shared__ unsigned long long wl[kQThreads / 32], wh[kQThreads / 32];
+  if ((threadIdx.x & 31) == 0) {
+    wl[threadIdx.x >> 5] = lo;
+    wh[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kQThreads / 32; w++) {
+      lo = min(lo, wl[w]);
+      hi = max(hi, wh[w]);
+    }
+    atomicMax(&head->neg_min, ~lo);
+    atomicMax(&head->max, hi);
   }
 }
 
-// One radix pass for a group of ranks: hist[g][bin] counts the keys whose bits
-// above `shift + 8` equal prefix[g], by their 8 bits at `shift`.  Lanes that
-// hit the same bin are combined before the shared-memory atomic.
-__global__ void __launch_bounds__(kQThreads) k_hist(const unsigned long long* __restrict__ keys, long long n, int shift,
-                                                    int nr, const unsigned long long* __restrict__ prefix,
-                                                    unsigned int* __restrict__ hist) {
-  __shared__ unsigned int sh[kGroup * 256];
-  __shared__ unsigned long long pf[kGroup];
-  for (int i = threadIdx.x; i < kGroup * 256; i += blockDim.x) sh[i] = 0;
-  if (threadIdx.x < nr) pf[threadIdx.x] = prefix[threadIdx.x];
+// True for the threads of the last block to arrive, which sees every other
+// block's writes.
+__device__ __forceinline__ bool last_block(unsigned int* ticket) {
+  __shared__ bool last;
+  __threadfence();
   __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// Executed by a warp: the bin of `hist` (in shared memory, a multiple of 32 bins)
+// that holds rank r; r becomes the rank within it, cnt its count.
+__device__ __forceinline__ int pick(const unsigned int* hist, int bins, unsigned long long& r, unsigned long long& cnt) {
+  const int lane = threadIdx.x & 31, per = bins / 32;
+  unsigned long long mine = 0;
+  for (int b = 0; b < per; b++) mine += hist[lane * per + b];
+  unsigned long long incl = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  // the first lane whose inclusive count exceeds r
+  const int src = __ffs(__ballot_sync(0xffffffffu, incl > r)) - 1;
+  int bin = 0;
+  unsigned long long rr = r, c = 0;
+  if (lane == src) {
+    rr -= incl - mine;
+    for (bin = lane * per;; bin++) {
+      c = hist[bin];
+      if (rr < c) break;
+      rr -= c;
+    }
+  }
+  r = __shfl_sync(0xffffffffu, rr, src);
+  cnt = __shfl_sync(0xffffffffu, c, src);
+  return __shfl_sync(0xffffffffu, bin, src);
+}
+
+// f(key, valid) for every key, by whole warps, four keys a lane loaded ahead.
+template <typename F>
+__device__ __forceinline__ void for_keys(const unsigned long long* __restrict__ keys, long long n, F&& f) {
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  // warp-uniform trip count: every lane runs the same number of iterations
-  const long long base0 = first - lane;
-  for (long long base = base0; base < n; base += stride) {
-    const long long i = base + lane;
-    const bool valid = i < n;
-    const unsigned long long key = valid ? keys[i] : 0ull;
-    const unsigned long long hi = shift >= 56 ? 0ull : (key >> (shift + 8));
-    const unsigned int bin = (unsigned int)(key >> shift) & 255u;
-    for (int g = 0; g < nr; g++) {
-      const bool m = valid && hi == pf[g];
-      if (!__any_sync(0xffffffffu, m)) continue;
-      const unsigned int peers = __match_any_sync(0xffffffffu, m ? bin : 0x100u + lane);
-      if (m && lane == __ffs(peers) - 1) atomicAdd(&sh[g * 256 + bin], (unsigned int)__popc(peers));
+  const long long stride = (long long)gridDim.x * kPassThreads * 4;
+  for (long long base = ((long long)blockIdx.x * kPassThreads + threadIdx.x - lane) * 4; base < n; base += stride) {
+    unsigned long long v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = base + 32 * u + lane < n ? keys[base + 32 * u + lane] : 0ull;
+#pragma unroll
+    for (int u = 0; u < 4; u++) f(v[u], base + 32 * u + lane < n);
+  }
+}
+
+// First pass of a group: a histogram over the keys' range, then every rank's bin.
+__global__ void __launch_bounds__(kPassThreads) k_select_first(const unsigned long long* __restrict__ keys, long long n,
+                                                              int bins, int nr, const __grid_constant__ QRanks ranks,
+                                                              const __grid_constant__ QLayout q) {
+  __shared__ unsigned int sh[kFirstMax];
+  const unsigned long long kmin = ~q.head->neg_min, range = q.head->max - kmin;
+  const int bits = 64 - __clzll((long long)range);
+  const int s1 = max(0, bits - (31 - __clz(bins)));
+  for (int i = threadIdx.x; i < bins; i += kPassThreads) sh[i] = 0;
+  __syncthreads();
+  for_keys(keys, n, [&](unsigned long long key, bool valid) {
+    if (valid) atomicAdd(&sh[(key - kmin) >> s1], 1u);
+  });
+  __syncthreads();
+  for (int i = threadIdx.x; i < bins; i += kPassThreads)
+    if (sh[i]) atomicAdd(&q.hist[i], sh[i]);
+  if (!last_block(&q.head->ticket)) return;
+  for (int i = threadIdx.x; i < bins; i += kPassThreads) sh[i] = __ldcg(&q.hist[i]);
+  __syncthreads();
+  const int w = threadIdx.x >> 5;
+  if (w < nr) {
+    unsigned long long r = ranks.r[w], c;
+    const int b = pick(sh, bins, r, c);
+    if ((threadIdx.x & 31) == 0) {
+      q.prefix[w] = (unsigned long long)b + (s1 == 0 ? kmin : 0ull);
+      q.rank[w] = r;
+      q.count[w] = c << 32 | c;
+      atomicOr(&q.map[b >> 5], 1u << (b & 31));
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nr * 256; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+  for (int i = threadIdx.x; i < max(bins, nr * kSub); i += kPassThreads) q.hist[i] = 0;
+  if (threadIdx.x == 0) {
+    q.head->ticket = 0;
+    q.head->todo = s1 == 0 ? 0ull : (1ull << nr) - 1ull;  // without lower bits a bin is one key
+    q.shifts[0] = q.shifts[1] = (unsigned int)s1;
+  }
 }
 
-// Picks, for every rank of the group, the bin that holds it: prefix gains the
-// bin's 8 bits and rank becomes the rank within the bin.
-__global__ void k_pick(int nr, unsigned long long* __restrict__ prefix, unsigned long long* __restrict__ rank,
-                       const unsigned int* __restrict__ hist) {
-  const int g = threadIdx.x;
-  if (g >= nr) return;
-  unsigned long long r = rank[g], below = 0;
-  int bin = 0;
-  for (; bin < 255; bin++) {
-    const unsigned long long c = hist[g * 256 + bin];
-    if (r < below + c) break;
-    below += c;
+// A later pass: the next bits of the keys in each open rank's bin; a bin of at
+// most kList keys is listed instead (in its counters' place), and the rank's key
+// taken from the list.
+__global__ void __launch_bounds__(kPassThreads) k_select_next(const unsigned long long* __restrict__ keys, long long n,
+                                                             int bins, int nr, const __grid_constant__ QLayout q) {
+  __shared__ unsigned int map[kFirstMax / 32];
+  __shared__ unsigned long long pf[kGroup], left;
+  __shared__ bool small[kGroup];
+  __shared__ __align__(8) unsigned int sh[kGroup * kSub];
+  const unsigned long long todo = q.head->todo;
+  if (todo == 0) return;  // the same for every block: an earlier launch wrote it
+  const unsigned long long kmin = ~q.head->neg_min;
+  const int s1 = (int)q.shifts[0], s = (int)q.shifts[1], d = min(s, kSubBits);
+  if (threadIdx.x < bins / 32) map[threadIdx.x] = q.map[threadIdx.x];
+  if (threadIdx.x < nr) {
+    pf[threadIdx.x] = q.prefix[threadIdx.x];
+    small[threadIdx.x] = (q.count[threadIdx.x] >> 32) <= kList;
   }
-  prefix[g] = (prefix[g] << 8) | (unsigned long long)bin;
-  rank[g] = r - below;
+  if (threadIdx.x == 0) left = todo;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for_keys(keys, n, [&](unsigned long long key, bool valid) {
+    const unsigned long long v = valid ? key - kmin : 0ull;
+    const unsigned int b = (unsigned int)(v >> s1);
+    const bool hit = valid && (map[b >> 5] >> (b & 31) & 1u);
+    if (!__any_sync(0xffffffffu, hit)) return;
+    const unsigned long long hi = v >> s;
+    for (int g = 0; g < nr; g++) {
+      const bool m = hit && (todo >> g & 1ull) && hi == pf[g];
+      if (!__any_sync(0xffffffffu, m)) continue;
+      if (small[g]) {
+        if (m) {
+          const unsigned int at = atomicAdd(reinterpret_cast<unsigned int*>(&q.count[g]), ~0u) - 1u;
+          reinterpret_cast<unsigned long long*>(q.hist + g * kSub)[at] = v + kmin;
+        }
+      } else {
+        const unsigned int bin = (unsigned int)(v >> (s - d)) & ((1u << d) - 1u);
+        const unsigned int peers = __match_any_sync(0xffffffffu, m ? bin : 0x1000u + lane);
+        if (m && lane == __ffs(peers) - 1) atomicAdd(&q.hist[g * kSub + bin], (unsigned int)__popc(peers));
+      }
+    }
+  });
+  if (!last_block(&q.head->ticket)) return;
+  for (int i = threadIdx.x; i < nr * kSub; i += kPassThreads) {
+    sh[i] = __ldcg(&q.hist[i]);
+    q.hist[i] = 0;
+  }
+  __syncthreads();
+  const int w = threadIdx.x >> 5;
+  if (w < nr && (todo >> w & 1ull)) {
+    unsigned long long r = q.rank[w];
+    if (small[w]) {  // the key with r others before it (equal keys in list order)
+      const unsigned long long* list = reinterpret_cast<const unsigned long long*>(sh + w * kSub);
+      const int c = (int)(__ldcg(&q.count[w]) >> 32);
+      for (int i = lane; i < c; i += 32) {
+        const unsigned long long x = list[i];
+        unsigned long long before = 0;
+        for (int j = 0; j < c; j++) {
+          const unsigned long long y = list[j];
+          before += y < x || (y == x && j < i);
+        }
+        if (before == r) q.prefix[w] = x;
+      }
+      if (lane == 0) atomicAnd(&left, ~(1ull << w));
+    } else {
+      unsigned long long c;
+      const int b = pick(sh + w * kSub, kSub, r, c);
+      if (lane == 0) {
+        const unsigned long long p = (pf[w] << d) | (unsigned long long)b;
+        q.prefix[w] = s == d ? p + kmin : p;
+        q.rank[w] = r;
+        q.count[w] = c << 32 | c;
+        if (s == d) atomicAnd(&left, ~(1ull << w));
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    q.head->ticket = 0;
+    q.head->todo = left;
+    q.shifts[1] = (unsigned int)(s - d);
+  }
 }
 
 }  // namespace
@@ -128,40 +353,59 @@ extern "C" int jne_percentiles_device(jne_context* c, const double* eigs_device,
   std::sort(ranks.begin(), ranks.end());
   ranks.erase(std::unique(ranks.begin(), ranks.end()), ranks.end());
   const int nr = (int)ranks.size();
-  // scratch: keys | NaN count | per rank: prefix, rank | histograms
-  const size_t words = (size_t)n + 1 + 2 * (size_t)nr + ((size_t)nr * 256 + 1) / 2;
+  // scratch: keys | head, shifts | per rank of a group: prefix, rank, count | map of first bins | histogram
+  const int ngmax = std::min(nr, kGroup), bins = first_bins(ngmax);
+  const size_t hist_words = (size_t)std::max(bins, ngmax * kSub) / 2, map_words = (size_t)bins / 64;
+  const size_t words = (size_t)n + kHeadWords + 3 * (size_t)ngmax + map_words + hist_words;
   if ((rc = ensure(c, &c->d_qscratch, &c->qscratch_cap, words, "percentile scratch"))) return rc;
   unsigned long long* keys = c->d_qscratch;
-  unsigned int* n_nan = reinterpret_cast<unsigned int*>(keys + n);
-  unsigned long long* prefix = keys + n + 1;
-  unsigned long long* rank = prefix + nr;
-  unsigned int* hist = reinterpret_cast<unsigned int*>(rank + nr);
+  QLayout q;
+  q.head = reinterpret_cast<QHead*>(keys + n);
+  q.shifts = reinterpret_cast<unsigned int*>(keys + n + kHeadWords - 1);
+  q.prefix = keys + n + kHeadWords;
+  q.rank = q.prefix + ngmax;
+  q.count = q.rank + ngmax;
+  q.map = reinterpret_cast<unsigned int*>(q.count + ngmax);
+  q.hist = q.map + 2 * map_words;
   cudaStream_t st = c->stream;
-  cudaError_t e = cudaMemsetAsync(n_nan, 0, sizeof(unsigned int), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(prefix, 0, sizeof(unsigned long long) * nr, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(rank, ranks.data(), sizeof(unsigned long long) * nr, cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaMemsetAsync(keys + n, 0, sizeof(unsigned long long) * (words - (size_t)n), st);
   if (e != cudaSuccess) return cuda_fail(c, e, "percentile setup");
   const long long want = (n + kQThreads - 1) / kQThreads;
   const int grid = (int)std::min<long long>(want, (long long)c->sms * 8);
-  k_aggregate<<<grid, kQThreads, 0, st>>>(eigs_device, n, k, stat, keys, n_nan);
-  for (int g0 = 0; g0 < nr && e == cudaSuccess; g0 += kGroup) {
-    const int ng = std::min(kGroup, nr - g0);
-    for (int pass = 0; pass < 8 && e == cudaSuccess; pass++) {
-      e = cudaMemsetAsync(hist, 0, sizeof(unsigned int) * 256 * ng, st);
-      if (e != cudaSuccess) break;
-      k_hist<<<grid, kQThreads, 0, st>>>(keys, n, 56 - 8 * pass, ng, prefix + g0, hist);
-      k_pick<<<1, kGroup, 0, st>>>(ng, prefix + g0, rank + g0, hist);
-      e = cudaGetLastError();
-    }
-  }
-  if (e != cudaSuccess) return cuda_fail(c, e, "percentile launch");
-  std::vector<unsigned long long> sel(nr);
+  // even rows of a 16-byte aligned table in 16-byte loads
+  if (k % 2 == 0 && reinterpret_cast<uintptr_t>(eigs_device) % 16 == 0)
+    k_aggregate<true><<<grid, kQThreads, 0, st>>>(eigs_device, n, k, stat, keys, q.head);
+  else
+    k_aggregate<false><<<grid, kQThreads, 0, st>>>(eigs_device, n, k, stat, keys, q.head);
+  const long long want_pass = (n + 4 * kPassThreads - 1) / (4 * kPassThreads);  // four keys a thread and round
+  const int grid_pass = (int)std::min<long long>(want_pass, (long long)c->sms * 2);
+  std::vector<unsigned long long> sel(nr), back(kHeadWords + (size_t)ngmax);
   unsigned int nans = 0;
-  e = cudaMemcpyAsync(sel.data(), prefix, sizeof(unsigned long long) * nr, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&nans, n_nan, sizeof nans, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return cuda_fail(c, e, "percentile select");
+  for (int g0 = 0; g0 < nr; g0 += kGroup) {
+    const int ng = std::min(kGroup, nr - g0);
+    QRanks gr{};
+    for (int g = 0; g < ng; g++) gr.r[g] = ranks[(size_t)(g0 + g)];
+    if (g0 > 0 && (e = cudaMemsetAsync(q.map, 0, sizeof(unsigned long long) * map_words, st)) != cudaSuccess)
+      return cuda_fail(c, e, "percentile setup");
+    k_select_first<<<grid_pass, kPassThreads, 0, st>>>(keys, n, bins, ng, gr, q);
+    unsigned long long todo = 1;
+    // at most 57 bits below the first digit, 7 a pass, and one more for a rank alone in its bin
+    for (int pass = 0; pass < 10 && todo; pass += 2) {
+      k_select_next<<<grid_pass, kPassThreads, 0, st>>>(keys, n, bins, ng, q);
+      k_select_next<<<grid_pass, kPassThreads, 0, st>>>(keys, n, bins, ng, q);
+      e = cudaGetLastError();
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(back.data(), q.head, sizeof(unsigned long long) * (kHeadWords + (size_t)ng),
+                            cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      if (e != cudaSuccess) return cuda_fail(c, e, "percentile select");
+      QHead head;
+      std::memcpy(&head, back.data(), sizeof head);
+      todo = head.todo;
+      nans = head.n_nan;
+    }
+    for (int g = 0; g < ng; g++) sel[(size_t)(g0 + g)] = back[kHeadWords + (size_t)g];
+  }
   if (nans) return fail(c, JNE_ERR_NUMERIC, std::to_string(nans) + " runs have a NaN aggregate (unordered)");
   auto at = [&](unsigned long long r) {
     const size_t i = (size_t)(std::lower_bound(ranks.begin(), ranks.end(), r) - ranks.begin());
