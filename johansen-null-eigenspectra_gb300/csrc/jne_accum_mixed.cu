@@ -28,6 +28,8 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
                          unsigned long long* __restrict__ counter, unsigned int* __restrict__ batch_done) {
   __shared__ WarpSmem sm_all[kMixWarps];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  if (lane == 0) sm_all[wib].slot_dim = 0;
+  __syncwarp();
   for (;;) {
     unsigned long long item = 0;
     if (lane == 0) item = atomicAdd(counter, 1ull);

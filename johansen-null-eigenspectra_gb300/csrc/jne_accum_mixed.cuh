@@ -391,20 +391,49 @@ __device__ __forceinline__ void tile_body(const float (*zs)[kZS], const float (*
 }
 
 // Per-warp shared memory of the accumulation (sized for the largest dim).
-constexpr int kRecMax = JNE_MAX_DIM * (JNE_MAX_DIM + 1) / 2 + 6 * JNE_MAX_DIM + JNE_MAX_DIM * JNE_MAX_DIM;
+constexpr int kProductSlots = JNE_MAX_DIM * (JNE_MAX_DIM + 1) / 2 + JNE_MAX_DIM * JNE_MAX_DIM;
+constexpr int kRecMax = kProductSlots + 6 * JNE_MAX_DIM;
 struct alignas(16) WarpSmem {
   float zs[16][kZS];      // increments of the current tile: z[feature][step]
   float bw[4][32];        // basis rows at the current tile's steps: 0, 1, u, u^2
   float cm[16][kCS];      // the chunk's local Gram, staged for the merge
   // float-float values are (hi, lo) pairs
   float2 wc[16];           // walk at the chunk start
-  float2 tz[16];           // chunk increment totals
   float2 rec[kRecMax];     // the run's record
   float2 mm[16];           // per feature: chunk mean m of the walk
-  float2 lm[16];           // Lc * m
-  float sbf[16], tzfs[16], cub[16], cuub[16], cuz[16], cuuz[16];
-  unsigned short mww_pr[JNE_MAX_DIM * (JNE_MAX_DIM + 1) / 2];
+  // walk (index f) and increment (16 + f) values side by side, so that one indexed form serves both
+  float2 lt[32];           // Lc * m | chunk increment totals
+  float st[32];            // sum b | total z
+  float cu[32], cuu[32];   // sum (u - ubar) b | z, sum ((u - ubar)^2 - qbar) b | z
+  uint2 slot[kProductSlots];  // operands of the product slots (see product_slot)
+  int slot_dim;            // dim the slot table was built for
 };
+
+// Which moments of the record a request's model needs beyond the products W W'
+// and z W': the sums of W (all but model 0), of y W and y z (models 2 to 4), of
+// y^2 W and y^2 z (model 4); everything for a pass that serves several models
+// (model < 0).  Returned as the number of d-slot kinds in the order of the merge:
+// W | y W, y z | y^2 W, y^2 z.
+__device__ __forceinline__ int moment_kinds(int model) { return model < 0 || model == 4 ? 5 : model == 0 ? 0 : model == 1 ? 1 : 3; }
+
+// Product slot t of a unit (each run's MWW entries, then its NzW): the index of
+// the left factor (walk 8 r + f, or 16 + 8 r + f for an increment), of the right,
+// walk factor, of the local Gram entry and of the record slot.
+template <int DIM, int NU>
+__device__ __forceinline__ uint2 product_slot(int t) {
+  constexpr int d = DIM, NMWW = d * (d + 1) / 2, NNZW = d * d, NREC = NMWW + NNZW + 6 * d;
+  if (t < NU * NMWW) {
+    const int r = t / NMWW, o = 8 * r;
+    int e = t - r * NMWW, p = 0;
+    while (e >= d - p) { e -= d - p; p++; }
+    const int c = p + e;
+    return make_uint2((uint32_t)(o + p) | (uint32_t)(o + c) << 16,
+                      (uint32_t)((o + p) * kCS + c) | (uint32_t)(r * NREC + t - r * NMWW) << 16);
+  }
+  const int u = t - NU * NMWW, r = u / NNZW, v = u - r * NNZW, za = v / d, wb = v - za * d, o = 8 * r;
+  return make_uint2((uint32_t)(16 + o + za) | (uint32_t)(o + wb) << 16,
+                    (uint32_t)((o + wb) * kCS + 16 + za) | (uint32_t)(r * NREC + NMWW + 3 * d + v) << 16);
+}
 
 // Lanes that own a walk feature in the merge: lane f < DIM, or (packed) lane
 // 8 r + f of run r.
@@ -432,28 +461,21 @@ __device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, Wa
   float (*zs)[kZS] = sm.zs;
   float (*cm)[kCS] = sm.cm;
   float2* wc = sm.wc;
-  float2* tz = sm.tz;
   float2* rec = sm.rec;
   float2* mm = sm.mm;
-  float2* lm = sm.lm;
-  float* sbf = sm.sbf;
-  float* tzfs = sm.tzfs;
-  float* cub = sm.cub;
-  float* cuub = sm.cuub;
-  float* cuz = sm.cuz;
-  float* cuuz = sm.cuuz;
-  unsigned short* mww_pr = sm.mww_pr;
+  float2* lt = sm.lt;
 
-  // staging rows without a feature stay zero; (p, r) of the walk moments
+  // staging rows without a feature stay zero
   for (int e = lane; e < 16 * kZS; e += 32) {
     const int row = e / kZS;
     if ((PAIR ? (row & 7) : row) >= d) (&zs[0][0])[e] = 0.f;
   }
-  for (int e = lane; e < NMWW; e += 32) {
-    int t = e, aa = 0;
-    while (t >= d - aa) { t -= d - aa; aa++; }
-    mww_pr[e] = (unsigned short)(aa | ((aa + t) << 8));
+  if (sm.slot_dim != (PAIR ? -d : d)) {  // once per warp, or when a ragged batch changes dim
+    for (int t = lane; t < NU * (NMWW + NNZW); t += 32) sm.slot[t] = product_slot<DIM, NU>(t);
+    __syncwarp();
+    if (lane == 0) sm.slot_dim = PAIR ? -d : d;
   }
+  const int kinds = moment_kinds(a.model);
   // G-row coefficients: value = c[0]*b + c[1] + c[2]*u + c[3]*u^2 (packed: the
   // lane's rows g and g + 8 are local row g of runs A and B)
   // the lane's rows: walk rows take c0 = 1 and the zero basis row (0); the basis rows take c0 = 0 and the
@@ -556,11 +578,11 @@ __device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, Wa
       float th, tl;
       if (g < d) {
         two_sum(chiA, cloA, th, tl);
-        tz[g] = make_float2(th, tl);
+        lt[16 + g] = make_float2(th, tl);
       }
       if (PAIR ? g < d : g + 8 < d) {
         two_sum(chiB, cloB, th, tl);
-        tz[g + 8] = make_float2(th, tl);
+        lt[24 + g] = make_float2(th, tl);
       }
     }
     __syncwarp();
@@ -596,60 +618,53 @@ __device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, Wa
       ff_mul(mh, ml, ct.lc, 0.f, ph, pe);
       float lh, ll = 0.f;
       two_sum(ph, pe, lh, ll);
-      lm[x] = make_float2(lh, ll);
-      const float tzf = tz[x].x;
-      sbf[x] = Sb;
-      tzfs[x] = tzf;
-      cub[x] = Sub - ub * Sb;                                              // sum (u-ubar) beta
-      cuub[x] = Suub - 2.0f * ub * Sub + ub * ub * Sb - Sb * invLcf * sig2;  // sum (u-ubar)^2 beta
-      cuz[x] = Suz - ub * tzf;                                             // sum (u-ubar) z
-      cuuz[x] = Suuz - 2.0f * ub * Suz + ub * ub * tzf - qbar * tzf;       // sum ((u-ubar)^2 - qbar) z
+      lt[x] = make_float2(lh, ll);
+      const float tzf = lt[16 + x].x;
+      sm.st[x] = Sb;
+      sm.st[16 + x] = tzf;
+      if (kinds > 0) {
+        sm.cu[x] = Sub - ub * Sb;                                               // sum (u-ubar) beta
+        sm.cuu[x] = Suub - 2.0f * ub * Sub + ub * ub * Sb - Sb * invLcf * sig2;   // sum (u-ubar)^2 beta
+        sm.cu[16 + x] = Suz - ub * tzf;                                          // sum (u-ubar) z
+        sm.cuu[16 + x] = Suuz - 2.0f * ub * Suz + ub * ub * tzf - qbar * tzf;    // sum ((u-ubar)^2 - qbar) z
+      }
     }
     __syncwarp();
-    // record slots, in order: MWW | MW1 MWy MWyy | NzW | Nz1 (from wc at the end) | Nzy Nzyy.
-    // One loop per slot kind, so the lanes of an iteration take one path.
-    const float c1y = hf, c2y = 2.0f * ybf * hf, c2yy = hf * hf;  // y and y^2 coefficients
-    for_slots<NU * NMWW, UNROLL>(lane, [&](int t) {
-      const int r = NU == 1 ? 0 : t / NMWW, e = t - r * NMWW, o = 8 * r;
-      const int p = o + (mww_pr[e] & 0xff), c = mww_pr[e] >> 8;
-      const float2 x = lm[p], y = mm[o + c];
+    // record slots, in two loops of one form each, so the lanes of an iteration take one path and few
+    // are idle (a slot is about 38 instructions; four loops, one per kind, left half the lanes of a small
+    // dim idle, and every moment was merged whatever the model; dim 2, T 1000, 100,000 runs of model 0: 1439 ->
+    // 1208 us, of model 4: 1506 -> 1360; dim 12, T 1000: model 0 6.89 -> 5.86 ms, model 3 7.34 -> 6.39).
+    // The products W W' and z W' (a mean product and the centred local part) ...
+    for_slots<NU * (NMWW + NNZW), UNROLL>(lane, [&](int t) {
+      const uint2 op = sm.slot[t];
+      const int x = op.x & 0xffff, w = op.x >> 16, e = op.y >> 16;
+      const float C = (&cm[0][0])[op.y & 0xffff];
+      const float2 xv = lt[x], yv = mm[w];
       float ph, pe;
-      ff_mul(x.x, x.y, y.x, y.y, ph, pe);
-      slot_acc(rec[r * NREC + e], ph, __fadd_rn(pe, cm[p][c] - sbf[p] * sbf[o + c] * invLcf));
+      ff_mul(xv.x, xv.y, yv.x, yv.y, ph, pe);
+      slot_acc(rec[e], ph, __fadd_rn(pe, C - sm.st[x] * sm.st[w] * invLcf));
     });
-    for_slots<NU * NMW, UNROLL>(lane, [&](int t) {
-      const int r = NU == 1 ? 0 : t / NMW, tt = t - r * NMW, pp = tt / d, x = 8 * r + tt - pp * d;
-      const int e = r * NREC + NMWW + tt;
+    // ... and the sums against 1, y and y^2 the model needs
+    const float c1y = hf, c2y = 2.0f * ybf * hf, c2yy = hf * hf;  // y and y^2 coefficients
+    const int n_sums = NU * d * kinds;
+    for_slots<NU * d * 5, UNROLL>(lane, [&](int t) {
+      if (t >= n_sums) return;
+      const int kind = t / (NU * d), v = t - kind * (NU * d), r = NU == 1 ? 0 : v / d, f = v - r * d;
+      const bool inc = kind == 2 || kind == 4;        // y z, y^2 z; else W, y W, y^2 W
+      const int pp = (kind + 1) >> 1, x = 8 * r + f + (inc ? 16 : 0);
+      const int e = r * NREC + (inc ? NMWW + NMW + NNZW : NMWW) + pp * d + f;
       const float wh = pp == 0 ? 1.f : pp == 1 ? ct.ybar_hi : ct.y2bar_hi;
       const float wl = pp == 0 ? 0.f : pp == 1 ? ct.ybar_lo : ct.y2bar_lo;
       const float a1 = pp == 0 ? 0.f : pp == 1 ? c1y : c2y, a2 = pp == 2 ? c2yy : 0.f;
       float ph, pe;
-      const float2 v = lm[x];
-      ff_mul(wh, wl, v.x, v.y, ph, pe);
-      slot_acc(rec[e], ph, __fadd_rn(pe, a1 * cub[x] + a2 * cuub[x]));
-    });
-    for_slots<NU * NNZW, UNROLL>(lane, [&](int t) {
-      const int r = NU == 1 ? 0 : t / NNZW, tt = t - r * NNZW, za = tt / d, wb = tt - za * d, o = 8 * r;
-      const int e = r * NREC + NMWW + NMW + tt;
-      float ph, pe;
-      const float2 x = tz[o + za], y = mm[o + wb];
-      ff_mul(x.x, x.y, y.x, y.y, ph, pe);
-      slot_acc(rec[e], ph, __fadd_rn(pe, cm[o + wb][16 + za] - tzfs[o + za] * sbf[o + wb] * invLcf));
-    });
-    for_slots<NU * 2 * d, UNROLL>(lane, [&](int t) {
-      const int r = NU == 1 ? 0 : t / (2 * d), tt = t - r * 2 * d, pp = tt / d, x = 8 * r + tt - pp * d;
-      const int e = r * NREC + NMWW + NMW + NNZW + d + tt;
-      const float wh = pp == 0 ? ct.ybar_hi : ct.y2bar_hi, wl = pp == 0 ? ct.ybar_lo : ct.y2bar_lo;
-      const float a1 = pp == 0 ? c1y : c2y, a2 = pp == 0 ? 0.f : c2yy;
-      float ph, pe;
-      const float2 v = tz[x];
-      ff_mul(wh, wl, v.x, v.y, ph, pe);
-      slot_acc(rec[e], ph, __fadd_rn(pe, a1 * cuz[x] + a2 * cuuz[x]));
+      const float2 xv = lt[x];
+      ff_mul(wh, wl, xv.x, xv.y, ph, pe);
+      slot_acc(rec[e], ph, __fadd_rn(pe, a1 * sm.cu[x] + a2 * sm.cuu[x]));
     });
     __syncwarp();
     if (lane_feature) {
       float2 w = wc[lane];
-      const float2 v = tz[lane];
+      const float2 v = lt[16 + lane];
       ff_acc(w.x, w.y, v.x, v.y);
       wc[lane] = w;
     }
@@ -717,6 +732,8 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, MINB)
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nwarps = gridDim.x * kMixWarps;
   const bool fused = fin.out != nullptr && a.batch_done != nullptr;
+  if (lane == 0) sm_all[wib].slot_dim = 0;
+  __syncwarp();
   const long long units = jne_units(DIM, a.n_runs, PACK);
   auto finalize_batch = [&](long long unit) {
     const long long first = batch_complete(a.batch_done, unit, units, lane);

@@ -186,7 +186,7 @@ int jne_eigs_seeded_models(jne_context* c, const int* models, int n_models, int 
       fa[m] = finalize_args(c, models[m], dim, steps, n, c->d_mom, c->d_out + off);
       off += (size_t)n * jne_eigen_count(models[m], dim);
     }
-    if ((rc = accumulate(c, models[0], dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
+    if ((rc = accumulate(c, n_models == 1 ? models[0] : -1, dim, steps, k0, k1, seed_first + (uint32_t)done, n, precision, nullptr,
                          c->d_mom, st, n_models == 1 ? fa : nullptr)))
       return rc;
     if (n_models > 1 && (rc = finalize(c, fa, n_models, st))) return rc;
