@@ -7,8 +7,10 @@
 
 namespace {
 
-// Blocks of two warps: few enough for the last wave to fill, and all models in
-// one grid, so that only the launch's own tail leaves SMs idle.
+// Blocks of two warps, and all models in one grid, so that only the launch's own
+// tail leaves SMs idle.  As many blocks per SM as registers allow: the local arrays
+// then miss L1, but the warps hide it (five models of 40,000 runs at k = 12, 13: 4.0
+// ms with 18 blocks per SM, 4.4 with 8, 5.2 with 4, 6.5 with 2).
 constexpr int kFinThreads = 64;
 
 struct FinalizeList {

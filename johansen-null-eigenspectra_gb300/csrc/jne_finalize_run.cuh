@@ -28,8 +28,9 @@
 // rank-two updates, the shift's correction in FP32 (any shift is a valid one: only
 // the convergence depends on it) and the deflation test on exponents.
 // Measured: five models of 40,000 runs at dim 12, T 2000 (one launch for all models
-// included) 11.25 -> 7.70 ms; 20,011 runs at dim 6, T 100, mostly finalize, 563 -> 447 us;
-// errors against quad precision no larger (dim 12, T 100, model 4: 4.1e-14 -> 2.3e-14 rms).
+// included) 11.25 -> 7.70 ms, and 6.9 with QL's sweeps in one loop; 20,011 runs at dim 6,
+// T 100, mostly finalize, 563 -> 447 -> 363 us; errors against quad precision no larger
+// (dim 12, T 100, model 4: 4.1e-14 -> 2.3e-14 rms).
 #pragma once
 #include <cfloat>
 #include <math_constants.h>
@@ -124,63 +125,69 @@ __device__ __forceinline__ bool is_zero(double x) { return ((__double2hiint(x) &
 // Eigenvalues of the symmetric tridiagonal matrix (dg, eo) by the implicit QL
 // method with Wilkinson shifts (Bowdler, Martin, Reinsch & Wilkinson, "The QR
 // and QL algorithms for symmetric matrices", Numer. Math. 11, 1968).  eo[i]
-// couples dg[i] and dg[i+1]; the iteration count per eigenvalue is bounded.
+// couples dg[i] and dg[i+1]; the sweep count per eigenvalue is bounded.  One loop
+// over sweeps, whichever eigenvalue a lane is at: the warp then runs as many as its
+// slowest lane in all, not the slowest lane's for each eigenvalue in turn.
 __device__ __forceinline__ bool tridiagonal_ql(double* dg, double* eo, int n) {
   eo[n - 1] = 0.0;
   bool ok = true;
-  for (int l = 0; l < n; l++) {
-    for (int iter = 0; iter < 64; iter++) {
-      int m = l;
+  int l = 0, sweeps = 0;
+  for (;;) {
+    int m = l;
+    for (; l < n; l++, sweeps = 0) {
       // negligible by exponents, with no FP64 instruction: |eo| < eps max(|dg[m]|, |dg[m + 1]|) when it
       // breaks, within a factor of four of |eo| <= eps (|dg[m]| + |dg[m + 1]|); never for a NaN
       int em = exponent_bits(dg[l]);
-      for (; m < n - 1; m++) {
+      for (m = l; m < n - 1; m++) {
         const int en = exponent_bits(dg[m + 1]);
         if (exponent_bits(eo[m]) <= max(em, en) - (53 << 20) || is_zero(eo[m])) break;
         em = en;
       }
-      if (m == l) break;
-      if (iter == 63) { ok = false; break; }
-      // the shift d_l - e_l / (g + sign(g) sqrt(g^2 + 1)), g = (d_{l+1} - d_l) / (2 e_l): its correction in FP32
-      const float ef = (float)eo[l], gf = (float)(dg[l + 1] - dg[l]) / (2.0f * ef);
-      double cf = (double)(ef / (gf + copysignf(sqrtf(fmaf(gf, gf, 1.0f)), gf)));
-      if (!isfinite(cf)) {  // values outside FP32's range
-        const double gd = (dg[l + 1] - dg[l]) / (2.0 * eo[l]);
-        cf = eo[l] / (gd + copysign(hypot(gd, 1.0), gd));
-      }
-      double g = dg[m] - dg[l] + cf;
-      double s = 1.0, c = 1.0, p = 0.0;
-      int i = m - 1;
-      bool underflow = false;
-      for (; i >= l; i--) {
-        const double f = s * eo[i], b = c * eo[i];
-        // Givens rotation from one reciprocal square root (the moments keep
-        // f and g far from the overflow / underflow range hypot guards)
-        const double r2 = fma(f, f, g * g);
-        if (r2 == 0.0) {  // recover from underflow
-          eo[i + 1] = 0.0;
-          dg[i + 1] -= p;
-          eo[m] = 0.0;
-          underflow = true;
-          break;
-        }
-        const double ir = rsqrt(r2);
-        eo[i + 1] = r2 * ir;
-        s = f * ir;
-        c = g * ir;
-        g = dg[i + 1] - p;
-        const double r = fma(dg[i] - g, s, 2.0 * c * b);
-        p = s * r;
-        dg[i + 1] = g + p;
-        g = fma(c, r, -b);
-      }
-      if (underflow) continue;
-      dg[l] -= p;
-      eo[l] = g;
-      eo[m] = 0.0;
+      if (m == l) continue;
+      if (sweeps < 63) break;
+      ok = false;  // not converged: on to the next eigenvalue
     }
+    if (l >= n) return ok;
+    sweeps++;
+    // the shift d_l - e_l / (g + sign(g) sqrt(g^2 + 1)), g = (d_{l+1} - d_l) / (2 e_l): its correction in FP32
+    const double dl = dg[l], el = eo[l];
+    const float ef = (float)el, gf = (float)(dg[l + 1] - dl) / (2.0f * ef);
+    double cf = (double)(ef / (gf + copysignf(sqrtf(fmaf(gf, gf, 1.0f)), gf)));
+    if (!isfinite(cf)) {  // values outside FP32's range
+      const double gd = (dg[l + 1] - dl) / (2.0 * el);
+      cf = el / (gd + copysign(hypot(gd, 1.0), gd));
+    }
+    double d1 = dg[m];  // dg[i + 1]
+    double g = d1 - dl + cf;
+    double s = 1.0, c = 1.0, p = 0.0;
+    int i = m - 1;
+    for (; i >= l; i--) {
+      const double e = eo[i], d0 = dg[i];
+      const double f = s * e, b = c * e;
+      // Givens rotation from one reciprocal square root (the moments keep
+      // f and g far from the overflow / underflow range hypot guards)
+      const double r2 = fma(f, f, g * g);
+      if (is_zero(r2)) break;  // underflow
+      const double ir = rsqrt(r2);
+      eo[i + 1] = r2 * ir;
+      s = f * ir;
+      c = g * ir;
+      g = d1 - p;
+      const double r = fma(d0 - g, s, 2.0 * c * b);
+      p = s * r;
+      dg[i + 1] = g + p;
+      g = fma(c, r, -b);
+      d1 = d0;
+    }
+    if (i >= l) {  // recover from underflow
+      eo[i + 1] = 0.0;
+      dg[i + 1] = d1 - p;
+    } else {
+      dg[l] = d1 - p;
+      eo[l] = g;
+    }
+    eo[m] = 0.0;
   }
-  return ok;
 }
 
 __device__ __noinline__ void finalize_run(const jne_finalize_args& f, int run) {
