@@ -720,6 +720,20 @@ int run_models(jne_context* ctx, const std::vector<int>& models, const std::vect
 
 }  // namespace
 
+namespace {
+
+// Puts v's order statistics ranks[a..b) (ascending, all within [lo, hi)) at their
+// places, given that v[lo..hi) holds the values of those places.
+void select_ranks(double* v, int64_t lo, int64_t hi, const int64_t* ranks, size_t a, size_t b) {
+  if (a >= b) return;
+  const size_t m = a + (b - a) / 2;
+  std::nth_element(v + lo, v + ranks[m], v + hi);
+  select_ranks(v, lo, ranks[m], ranks, a, m);
+  select_ranks(v, ranks[m] + 1, hi, ranks, m + 1, b);
+}
+
+}  // namespace
+
 extern "C" {
 
 int jne_simulation_run(jne_context* ctx, const char* data_dir, int model, int dim, int steps, int64_t num_runs,
@@ -779,7 +793,17 @@ int jne_percentiles(const double* eigs, int64_t n, int k, int stat, const double
   }
   // the reference's sort (partial_cmp().unwrap(), simulation_analyzers.rs:60) panics on NaN
   if (nans) return dat_fail(JNE_ERR_NUMERIC, std::to_string(nans) + " runs have a NaN aggregate (unordered)");
-  std::sort(v.begin(), v.end());
+  // only the order statistics next to the wanted ranks: each selected within the range its neighbours left, halving
+  // the list of ranks (200,000 x 5 values, 7 percentiles, the sums included: 3.6 ms, sorted 10.6)
+  std::vector<int64_t> ranks;
+  for (int i = 0; i < np && n > 0; i++) {
+    const double rank = ps[i] * (double)(n - 1);
+    ranks.push_back((int64_t)std::floor(rank));
+    ranks.push_back((int64_t)std::ceil(rank));
+  }
+  std::sort(ranks.begin(), ranks.end());
+  ranks.erase(std::unique(ranks.begin(), ranks.end()), ranks.end());
+  select_ranks(v.data(), 0, n, ranks.data(), 0, ranks.size());
   for (int i = 0; i < np; i++) {  // simulation_analyzers.rs:4-18
     if (n == 0) {
       out[i] = NAN;
