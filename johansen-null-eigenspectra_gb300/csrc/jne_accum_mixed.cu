@@ -30,11 +30,11 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   if (lane == 0) sm_all[wib].slot_dim = 0;
   __syncwarp();
-  for (;;) {
-    unsigned long long item = 0;
-    if (lane == 0) item = atomicAdd(counter, 1ull);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= (unsigned long long)total) break;
+  // first item by warp, then the next free one from the counter: the warps of a block run the same dim's code
+  // (the launch's items are ordered by dim), which fits the instruction cache where several dims' does not
+  const unsigned long long nwarps = (unsigned long long)gridDim.x * kMixWarps;
+  for (unsigned long long item = (unsigned long long)blockIdx.x * kMixWarps + wib;
+       item < (unsigned long long)total;) {
     const int lo = request_of(reqs, n_req, (long long)item);
     const jne_accum_args& a = reqs[lo].acc;
     const int unit = (int)(item - (unsigned long long)reqs[lo].first);
@@ -61,6 +61,9 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
       }
       __syncwarp();
     }
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(counter, 1ull);
+    item = nwarps + __shfl_sync(0xffffffffu, next, 0);
   }
 }
 
