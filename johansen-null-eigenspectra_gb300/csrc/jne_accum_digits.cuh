@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 3)
     digit_unit<DIM, true>(a, (int)unit, sm_all[wib], rk, lane);
     if (fused) {
       const long long first = batch_complete(a.batch_done, unit, units, lane);
-      if (first >= 0 && first + lane < units) finalize_unit(fin, first + lane, true);
+      if (first >= 0) finalize_batch(fin, first, true, lane);
       __syncwarp();
     }
     unsigned long long item = 0;

@@ -55,9 +55,29 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
     }
     if (batch_done) {
       const long long first = batch_complete(batch_done, (long long)item, total, lane);
-      if (first >= 0 && first + lane < total) {
-        const int r = request_of(reqs, n_req, first + lane);
-        finalize_unit(reqs[r].fin, first + lane - reqs[r].first, true);
+      if (first >= 0) {
+        // one run per lane; batches of packed pairs in two rounds of 16 items, batches that mix packed and
+        // unpacked dims one item per lane
+        const bool mine = first + lane < total;
+        const int r0 = mine ? request_of(reqs, n_req, first + lane) : 0;
+        const bool packed = !mine || reqs[r0].acc.dim <= JNE_PACK_MAX_DIM;
+        if (__all_sync(0xffffffffu, packed)) {
+          for (int s = lane; s < 64; s += 32) {
+            const long long it = first + (s >> 1);
+            if (it < total) {
+              const jne_ragged_req& q = reqs[request_of(reqs, n_req, it)];
+              const long long run = 2 * (it - q.first) + (s & 1);
+              if (run < q.fin.n_runs) jne_fin::finalize_run(q.fin, (int)run);
+            }
+          }
+        } else if (mine) {
+          const jne_ragged_req& q = reqs[r0];
+          const int nu = packed ? 2 : 1;
+          for (int u = 0; u < nu; u++) {
+            const long long run = nu * (first + lane - q.first) + u;
+            if (run < q.fin.n_runs) jne_fin::finalize_run(q.fin, (int)run);
+          }
+        }
       }
       __syncwarp();
     }

@@ -708,13 +708,13 @@ __device__ __forceinline__ long long batch_complete(unsigned int* batch_done, lo
   return first;
 }
 
-// The finalize of one unit's runs (one, or a packed pair).
-__device__ __forceinline__ void finalize_unit(const jne_finalize_args& fin, long long unit, bool pack) {
+// The finalize of a request's batch: units first .. first + 31, one run per lane
+// (packed pairs: 64 runs in two rounds of neighbours, so that a short batch keeps
+// its runs in different lanes and the record reads stay contiguous).
+__device__ __forceinline__ void finalize_batch(const jne_finalize_args& fin, long long first, bool pack, int lane) {
   const int nu = pack && fin.dim <= JNE_PACK_MAX_DIM ? 2 : 1;
-  for (int r = 0; r < nu; r++) {
-    const long long run = nu * unit + r;
-    if (run < fin.n_runs) jne_fin::finalize_run(fin, (int)run);
-  }
+  const long long end = min((long long)fin.n_runs, nu * (first + 32));
+  for (long long run = nu * first + lane; run < end; run += 32) jne_fin::finalize_run(fin, (int)run);
 }
 
 // One request: every warp strides over its units.  The round keys arrive as a
@@ -735,21 +735,21 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, MINB)
   if (lane == 0) sm_all[wib].slot_dim = 0;
   __syncwarp();
   const long long units = jne_units(DIM, a.n_runs, PACK);
-  auto finalize_batch = [&](long long unit) {
+  auto finalize_done = [&](long long unit) {
     const long long first = batch_complete(a.batch_done, unit, units, lane);
-    if (first >= 0 && first + lane < units) finalize_unit(fin, first + lane, PACK);
+    if (first >= 0) finalize_batch(fin, first, PACK, lane);
     __syncwarp();
   };
   if (a.next_run == nullptr) {
     for (long long unit = blockIdx.x * kMixWarps + wib; unit < units; unit += nwarps) {
       accum_unit<DIM, EXT, true, PACK>(a, (int)unit, sm_all[wib], rk, lane);
-      if (fused) finalize_batch(unit);
+      if (fused) finalize_done(unit);
     }
   } else {
     // first unit by warp index, then the next free one from the counter
     for (long long unit = blockIdx.x * kMixWarps + wib; unit < units;) {
       accum_unit<DIM, EXT, true, PACK>(a, (int)unit, sm_all[wib], rk, lane);
-      if (fused) finalize_batch(unit);
+      if (fused) finalize_done(unit);
       unsigned long long item = 0;
       if (lane == 0) item = atomicAdd(a.next_run, 1ull);
       unit = nwarps + (long long)__shfl_sync(0xffffffffu, item, 0);
