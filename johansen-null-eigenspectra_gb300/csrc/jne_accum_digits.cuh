@@ -520,7 +520,7 @@ __device__ __forceinline__ void digit_unit(const jne_accum_args& a, int unit, Di
   __syncwarp();
 }
 
-template <int DIM>
+template <int DIM, bool PACK>
 __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 3)
     k_accum_digits(const __grid_constant__ jne_accum_args a, const __grid_constant__ jne_round_keys rk,
                    const __grid_constant__ jne_finalize_args fin) {
@@ -528,13 +528,13 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 3)
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nwarps = gridDim.x * kMixWarps;
   const bool fused = fin.out != nullptr && a.batch_done != nullptr;
-  const long long units = jne_units(DIM, a.n_runs, true);
+  const long long units = jne_units(DIM, a.n_runs, PACK);
   // first unit by warp index, then the next free one from the counter
   for (long long unit = blockIdx.x * kMixWarps + wib; unit < units;) {
-    digit_unit<DIM, true>(a, (int)unit, sm_all[wib], rk, lane);
+    digit_unit<DIM, PACK>(a, (int)unit, sm_all[wib], rk, lane);
     if (fused) {
       const long long first = batch_complete(a.batch_done, unit, units, lane);
-      if (first >= 0) finalize_batch(fin, first, true, lane);
+      if (first >= 0) finalize_batch(fin, first, PACK, lane);
       __syncwarp();
     }
     unsigned long long item = 0;
@@ -546,8 +546,10 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 3)
 template <int DIM>
 cudaError_t launch_digits_dim(const jne_accum_args& a, const jne_finalize_args& fin, int sms, cudaStream_t st) {
   const int threads = kMixWarps * JNE_WARP;
-  auto k = k_accum_digits<DIM>;
-  k<<<resident_grid(k, threads, 0, sms, jne_units(DIM, a.n_runs, true), kMixWarps), threads, 0, st>>>(
+  // small dims pack two runs per warp once every run can no longer have a warp of its own (3 blocks of 4 per SM)
+  const bool pack = DIM <= JNE_PACK_MAX_DIM && a.n_runs > 12 * sms;
+  auto k = pack ? k_accum_digits<DIM, (DIM <= JNE_PACK_MAX_DIM)> : k_accum_digits<DIM, false>;
+  k<<<resident_grid(k, threads, 0, sms, jne_units(DIM, a.n_runs, pack), kMixWarps), threads, 0, st>>>(
       a, jne_make_round_keys(a.key0, a.key1), fin);
   return cudaGetLastError();
 }
