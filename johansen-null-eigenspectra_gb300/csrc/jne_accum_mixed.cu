@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
             if (it < total) {
               const jne_ragged_req& q = reqs[request_of(reqs, n_req, it)];
               const long long run = 2 * (it - q.first) + (s & 1);
-              if (run < q.fin.n_runs) jne_fin::finalize_run(q.fin, (int)run);
+              if (run < q.fin.n_runs) jne_fin::finalize_run<false>(q.fin, (int)run);
             }
           }
         } else if (mine) {
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
           const int nu = packed ? 2 : 1;
           for (int u = 0; u < nu; u++) {
             const long long run = nu * (first + lane - q.first) + u;
-            if (run < q.fin.n_runs) jne_fin::finalize_run(q.fin, (int)run);
+            if (run < q.fin.n_runs) jne_fin::finalize_run<false>(q.fin, (int)run);
           }
         }
       }

@@ -714,7 +714,7 @@ __device__ __forceinline__ long long batch_complete(unsigned int* batch_done, lo
 __device__ __forceinline__ void finalize_batch(const jne_finalize_args& fin, long long first, bool pack, int lane) {
   const int nu = pack && fin.dim <= JNE_PACK_MAX_DIM ? 2 : 1;
   const long long end = min((long long)fin.n_runs, nu * (first + 32));
-  for (long long run = nu * first + lane; run < end; run += 32) jne_fin::finalize_run(fin, (int)run);
+  for (long long run = nu * first + lane; run < end; run += 32) jne_fin::finalize_run<false>(fin, (int)run);
 }
 
 // One request: every warp strides over its units.  The round keys arrive as a

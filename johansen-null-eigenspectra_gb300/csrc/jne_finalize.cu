@@ -20,7 +20,7 @@ struct FinalizeList {
 __global__ void __launch_bounds__(kFinThreads) k_finalize(const __grid_constant__ FinalizeList list) {
   const jne_finalize_args& f = list.f[blockIdx.y];
   const int run = blockIdx.x * kFinThreads + threadIdx.x;
-  if (run < f.n_runs) jne_fin::finalize_run(f, run);
+  if (run < f.n_runs) jne_fin::finalize_run<true>(f, run);
 }
 
 }  // namespace
