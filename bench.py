@@ -8,7 +8,7 @@ FP32 chunks, float-float merge and FP64 Cholesky + tridiagonal QL).
 
   value   runs/s with results left in device memory (jne_eigs_seeded_device)
   e2e     runs/s through jne_eigs_seeded: eigenvalues copied to host memory
-  fp64_plain  runs/s of the plain FP64 fused kernel on the same workload
+  fp64_plain  runs/s of the FP64 form on the same workload
   mixed_error max relative max-eig / trace error of mixed vs FP64 on identical seeds
 
 `--impl reference` times the CPU restatement of the reference algorithm (the
@@ -39,13 +39,13 @@ UNIT = "runs/s"
 
 # DRAM bytes (read + write) of one k_accum_mixed<12> launch (accumulation + fused
 # finalize) per run, from an ncu capture of the full 200,000-run launch
-# (profiles/k_accum_mixed_dim12_T10k_dram.md): 18,147,072 B read + 771,372,800 B written.
+# (profiles/k_accum_mixed_dim12_T10k_dram.md): 19,942,912 B read + 625,956,352 B written.
 # Algorithmic: 2,352 B of record written and read back, 96 B of eigenvalues per run.
-ACCUM_DRAM_BYTES_PER_RUN = (18_147_072 + 771_372_800) / 200_000
+ACCUM_DRAM_BYTES_PER_RUN = (19_942_912 + 625_956_352) / 200_000
 # Warp instructions k_accum_mixed<12> issues per run at T = 10,000 (accumulation plus
 # the run's share of its fused finalize batch), from an ncu capture of an 8,192-run
-# launch (profiles/k_accum_mixed_dim12_T10k_8192runs_full.md): 1,166,615,378 / 8,192.
-ACCUM_WARP_INST_PER_RUN = 142_409
+# launch (profiles/k_accum_mixed_dim12_T10k_8192runs_full.md): 1,150,649,595 / 8,192.
+ACCUM_WARP_INST_PER_RUN = 140_460
 
 
 def k_of(model: int) -> int:
@@ -197,8 +197,7 @@ def run_gpu(args, rank: int, world: int) -> None:
     seed0 = replica_seed_first(rank, R)
     stream = torch.cuda.Stream()
     sptr = stream.cuda_stream
-    # requests alternate between two caller streams, so the finalize of one
-    # request (on the engine's second stream) overlaps the next accumulation
+    # requests alternate between two caller streams (the engine runs them in order on its own)
     streams = [stream, torch.cuda.Stream()]
     outs = {m: torch.empty((R, k_of(m)), dtype=torch.float64, device="cuda") for m in MODELS}
 
@@ -278,7 +277,7 @@ def run_gpu(args, rank: int, world: int) -> None:
     e2e = runs_per_step * args.steps / e2e_s
     d2h = sum(R * k_of(m) * 8 for m in MODELS)
 
-    # ---- plain FP64 fused kernel on the same workload (fewer runs) ----
+    # ---- the FP64 form on the same workload (fewer runs) ----
     Rf = args.fp64_runs
     for m in MODELS:
         eng.eigs_seeded_device(m, DIM, STEPS, seed0, Rf, outs[m].data_ptr(), precision=jne.PREC_FP64, stream=sptr)
@@ -411,7 +410,7 @@ def run_gpu(args, rank: int, world: int) -> None:
                            "step": "5 requests, one per model, pipelined"},
             "fp64_plain": {"value": fp64_value, "unit": UNIT, "runs_per_model": Rf,
                            "mixed_speedup": value / fp64_value},
-            "mixed_error": {"vs": "plain FP64 kernel, identical seeds", "runs_per_model": ns, "per_model": err},
+            "mixed_error": {"vs": "FP64 form, identical seeds", "runs_per_model": ns, "per_model": err},
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": d2h},
             "gpu_launches": acc_n + fin_n,
             "roofline": roof, "issue_bound": issue, "kernel_ms": kern,
@@ -516,7 +515,7 @@ def bench_ragged60(jne, torch, local: int, steps: int, tune: float = 0.0) -> dic
 
 def bench_precision(jne, torch, local: int, runs: int, subset: int = 10_000) -> dict:
     """Model 4, dim 12, T 1e4: `runs` runs in mixed precision (device outputs), and the max-eig / trace error
-    of the first `subset` of them against the plain FP64 kernel on the same seeds."""
+    of the first `subset` of them against the FP64 form on the same seeds."""
     k = jne.eigen_count(4, DIM)
     out = torch.empty((runs, k), dtype=torch.float64, device="cuda")
     with jne.Engine(local) as eng:
@@ -544,7 +543,7 @@ def bench_precision(jne, torch, local: int, runs: int, subset: int = 10_000) -> 
             "trace_rel_err": {"max": float(rel_tr.max()), "p99": float(np.percentile(rel_tr, 99)),
                               "mean": float(rel_tr.mean())},
             "workload": f"model 4, dim {DIM}, T {STEPS}, {runs} runs mixed (seeds 1..{runs}); error of the first "
-                        f"{ns} vs the plain FP64 kernel on the same seeds"}
+                        f"{ns} vs the FP64 form on the same seeds"}
 
 
 def precision_vs_oracle(jne, local: int, oracle, runs: int, threads: int) -> dict:
