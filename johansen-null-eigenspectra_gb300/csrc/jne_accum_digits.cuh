@@ -39,7 +39,8 @@
 // with FP64 multiply-adds (one warp per run, 7-9 table entries per lane), 5.78 ms
 // in digits; dim 5, T 1000, 50,001 runs: 9.62 -> 2.07 ms.  Errors against quad
 // precision (normwise, rms over runs, dim 12): model 1, T 10^4 2.6e-12 -> 9.3e-15,
-// T 1000 5.5e-14 -> 7.8e-15, T 32 5.5e-15 -> 4.5e-15.
+// T 1000 5.5e-14 -> 7.8e-15, T 33 6.2e-15 -> 4.4e-15; shorter paths keep the
+// multiply-adds (jne_accum_digits.cu).
 // What bounds it now: 98 MMAs per 32-step tile (784 cycles), beside which the digit
 // extraction's integer instructions (2 cycles each) and the Philox multiplies (3.3)
 // hardly run.  Registers: 72 accumulators; 3 blocks of 4 warps per SM (168
@@ -409,9 +410,8 @@ __device__ __forceinline__ void digit_unit(const jne_accum_args& a, int unit, Di
     const int Lc = min(t0, T) - c0;
     const int ntile = (t0 - c0) >> 5;
     // the squares of d3 left out with G_6 have a mean too, (1024^2 - 1) / 12 for every step but the chunk's first
-    // (b = 0): 256/3 in units of G_5.  Not on paths so short that S11 may be singular: there its rounding should
-    // not be lifted above zero.
-    const int left_out = T > JNE_MAX_K + 3 ? ((Lc - 1) * 256 + 1) / 3 : 0;
+    // (b = 0): 256/3 in units of G_5.
+    const int left_out = ((Lc - 1) * 256 + 1) / 3;
 
     // ---- chunk end: the local Gram, staged in FP64 (cm[row][col], as in the mixed kernel: col < 16 walk columns,
     //      16 + f increments).  Symmetric blocks are staged doubled, their transposes added by the merge. ----

@@ -7,6 +7,7 @@
 #define JNE_MAX_DIM 12
 #define JNE_MAX_K 13
 #define JNE_WARP 32
+#define JNE_SHORT_STEPS 32 /* FP64: paths of at most this many steps (one tile) are summed in multiply-adds */
 
 // ---------------------------------------------------------------------------
 // Counter-based increments (Philox4x32-10, Salmon et al., SC'11).
