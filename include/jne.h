@@ -49,7 +49,8 @@ extern "C" {
 
 /* arithmetic of the Gram contraction */
 /* plain form: exact Gram sums (digits of the engine's increments on the tensor
- * cores; FP64 multiply-adds for explicit increments), FP64 record and solve */
+ * cores; FP64 multiply-adds for explicit increments and for paths of at most 32
+ * steps), FP64 record and solve */
 #define JNE_PREC_FP64 0
 #define JNE_PREC_MIXED 1 /* split FP16/TF32 tensor-core Grams, FP32 chunks, float-float merge, FP64 solve */
 /* JNE_PREC_MIXED requests with fewer steps than this run the FP64 kernel: on
