@@ -37,6 +37,7 @@ __host__ __device__ __forceinline__ jne_round_keys jne_make_round_keys(uint32_t 
   return rk;
 }
 
+#ifdef __CUDACC__  // device code; the declarations around it serve host compilers too
 // Ten rounds of the multiply/xor bijection; each 32x32->64 product yields both
 // halves at once.
 __device__ __forceinline__ void jne_philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
@@ -123,6 +124,8 @@ __device__ __forceinline__ void jne_normal_quad(uint32_t s, uint32_t j, uint32_t
   z[2] = z23.x;
   z[3] = z23.y;
 }
+
+#endif  // __CUDACC__
 
 // ---------------------------------------------------------------------------
 // Per-run moment record (FP64), in units of the unscaled walk W_i = sum_{s<=i} z_s

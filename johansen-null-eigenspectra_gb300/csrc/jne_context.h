@@ -336,6 +336,7 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
   if (precision == JNE_PREC_FP64 && d_ext) {  // explicit increments: FP64 multiply-adds
     if (c->ent_model != model || c->ent_dim != dim) {
       int4 host_ent[512];
+      c->ent_model = -2;  // until the upload: a failure must not leave the old key over a lost table
       c->ent_n = jne_build_f64_entries(model, dim, host_ent, 512);
       int rc = ensure(c, &c->d_ent, &c->ent_cap, 512, "entry table");
       if (rc) return rc;
@@ -355,6 +356,7 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
     // per-chunk time means, exact (integer sums) then rounded once
     const int nch = (steps + a.chunk - 1) / a.chunk;
     if (c->ctab_steps != steps || c->ctab_chunk != a.chunk) {
+      c->ctab_steps = -1;  // as above
       int rc = ensure(c, &c->d_ctab, &c->ctab_cap, (size_t)nch, "chunk table");
       if (rc) return rc;
       c->h_ctab.resize(nch);
