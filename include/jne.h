@@ -84,10 +84,12 @@ const char* jne_last_error(const jne_context* ctx);
 int jne_set_chunk(jne_context* ctx, int chunk);
 
 /* The mixed single-request kernel's variant outside JNE_CHUNK_TUNED mode:
- * blocks_per_sm 4 (the default, 128 registers a thread) or 6 (80), and for
- * dims up to 4 pack = 1 (the default, two runs per warp) or 0 (one).  0 for
- * either keeps its default.  Speed only: every variant gives the same bits.
- * No counterpart in the reference. */
+ * blocks_per_sm 4 (the default, also as 0; 128 registers a thread) or 6 (80),
+ * and for dims up to 4 pack = 1 (two runs per warp) or 0 (one) whatever the
+ * request's size.  A context on which this was never called packs requests of
+ * more than 16 runs per SM only: fewer runs each have a warp of their own.
+ * Speed only: every variant gives the same bits.  No counterpart in the
+ * reference. */
 int jne_set_launch_shape(jne_context* ctx, int blocks_per_sm, int pack);
 
 /* One candidate launch shape of the mixed kernel, as jne_autotune measured it. */
@@ -107,8 +109,9 @@ typedef struct jne_tune_entry {
  * to the first over max_rel_err; then it times, with CUDA events, one launch of
  * time_runs runs (0: sized for about 20-60 ms) for every shape of every chunk
  * within the bound: blocks per SM 4 or 6, and one or two runs per warp for dims
- * up to 4.  The fastest shape is stored in ctx for JNE_CHUNK_TUNED and written
- * to *chosen; the measured candidates go to table (up to table_cap, *n_table of
+ * up to 4.  The fastest shape is stored in ctx for JNE_CHUNK_TUNED (its packing
+ * only where it differs from what the size rule of jne_set_launch_shape takes at
+ * time_runs) and written to *chosen; the measured candidates go to table (up to table_cap, *n_table of
  * them).  Only the chunk changes results: shapes of one chunk give the same
  * bits.  Classes below JNE_MIXED_MIN_STEPS run the FP64 kernel and are not
  * tuned (JNE_ERR_ARG).  table, n_table and chosen may be null. */

@@ -775,14 +775,10 @@ template <int DIM, int MINB, bool EXT>
 cudaError_t launch_dim(const jne_accum_args& a, const jne_finalize_args& fin, int sms, cudaStream_t st) {
   const int threads = kMixWarps * JNE_WARP;
   const jne_round_keys rk = jne_make_round_keys(a.key0, a.key1);
-  // one run per warp while every run has a warp of its own (4 blocks of 4 warps per SM): packed, half the warps
-  // would do twice the work (608 runs: dim 2, T 1000 106 -> 77 us, dim 4 210 -> 129, dim 3, T 10^4 284 -> 199; equal
-  // at 2,432 runs, and 1.3x the other way at 4,864)
-  const bool pack = a.pack >= 0 && a.n_runs > 16 * sms;
   if (EXT) {
     auto k = k_accum_mixed<DIM, true, MINB, true>;
     k<<<resident_grid(k, threads, 0, sms, jne_units(DIM, a.n_runs, true), kMixWarps), threads, 0, st>>>(a, rk, fin);
-  } else if (pack || DIM > JNE_PACK_MAX_DIM) {
+  } else if (a.pack >= 0 || DIM > JNE_PACK_MAX_DIM) {
     auto k = k_accum_mixed<DIM, false, MINB, true>;
     k<<<resident_grid(k, threads, 0, sms, jne_units(DIM, a.n_runs, true), kMixWarps), threads, 0, st>>>(a, rk, fin);
   } else {

@@ -13,9 +13,10 @@
 
 // The mixed kernel's launch shape for one (dim, class of steps): chunk length,
 // blocks per SM of the kernel variant (4 or 6) and whether dims <= 4 pack two
-// runs per warp.  Only the chunk changes the arithmetic.
+// runs per warp: 1, 0, or -1 for jne_pack_by_default.  Only the chunk changes the
+// arithmetic.
 struct jne_shape {
-  int chunk = 0, blocks_per_sm = 4, pack = 1;
+  int chunk = 0, blocks_per_sm = 4, pack = -1;
 };
 
 struct jne_context {
@@ -207,8 +208,9 @@ inline int chunk_for(const jne_context* c, int dim, int steps) {
 }
 
 // The single-request kernel variant for (dim, steps): the tuned one in
-// JNE_CHUNK_TUNED mode, else 4 blocks per SM with packed small dims (or the
-// tuner's candidate while it times one).
+// JNE_CHUNK_TUNED mode, else the caller's (jne_set_launch_shape) or the
+// default: 4 blocks per SM, small dims packed by the size rule (or the tuner's
+// candidate while it times one).
 inline jne_shape shape_for(const jne_context* c, int dim, int steps) {
   jne_shape s = c->force;
   if (c->chunk == JNE_CHUNK_TUNED) {
@@ -369,7 +371,8 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
     a.chunk_tab = c->d_ctab;
     const jne_shape shape = shape_for(c, dim, steps);
     a.blocks_per_sm = d_ext ? 4 : shape.blocks_per_sm;
-    a.pack = d_ext || shape.pack ? 0 : -1;
+    const bool pack = shape.pack < 0 ? jne_pack_by_default(n, c->sms) : shape.pack != 0;
+    a.pack = d_ext || pack ? 0 : -1;
   }
   // warps take runs from a counter, so warps that start late or finalize take fewer
   e = cudaMemsetAsync(c->d_next_run, 0, sizeof(unsigned long long), st);

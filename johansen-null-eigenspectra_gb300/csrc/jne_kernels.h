@@ -18,6 +18,12 @@ __host__ __device__ __forceinline__ long long jne_units(int dim, long long n_run
   return pack && dim <= JNE_PACK_MAX_DIM ? (n_runs + 1) / 2 : n_runs;
 }
 
+// Whether the mixed single-request kernel packs when nobody chose: one run per warp
+// while every run has a warp of its own (4 blocks of 4 warps per SM); packed, half the
+// warps would do twice the work (608 runs: dim 2, T 1000 106 -> 77 us, dim 4 210 -> 129,
+// dim 3, T 10^4 284 -> 199; equal at 2,432 runs, and 1.3x the other way at 4,864).
+inline bool jne_pack_by_default(long long n_runs, int sms) { return n_runs > 16ll * sms; }
+
 // Argument block of the finalize kernel.
 struct jne_finalize_args {
   int model, dim, steps, n_runs;

@@ -1,0 +1,68 @@
+// The launch shape a mixed request reaches its kernel with: the size rule by default, the caller's packing at every
+// size, and what the tuner times and keeps on either side of the rule's line.
+#include "fake_cuda.h"
+
+#include <cstdio>
+
+cudaError_t jne_launch_export(int, int, int, uint32_t, uint32_t, uint32_t, double, double*, uint32_t*, cudaStream_t) {
+  return cudaSuccess;
+}
+int jne_build_f64_entries(int, int, int4*, int) { return 0; }
+
+namespace {
+
+int failures = 0;
+void check(bool ok, const char* what, long long x = 0, long long y = 0) {
+  if (!ok) {
+    failures++;
+    std::printf("FAILED: %s (%lld, %lld)\n", what, x, y);
+  }
+}
+
+bool packed(jne_context* c, int dim, int64_t n) {
+  std::vector<double> out((size_t)n * jne_eigen_count(0, dim));
+  check(jne_eigs_seeded(c, 0, dim, 1000, 1, 1, n, JNE_PREC_MIXED, out.data()) == JNE_OK, "request");
+  return fake::mixed.back().a.pack >= 0;
+}
+
+}  // namespace
+
+int main() {
+  const int64_t line = 16 * fake::kSms;
+  for (int dim = 1; dim <= JNE_PACK_MAX_DIM; dim++) {
+    jne_context* c = nullptr;
+    check(jne_open(0, 0, &c) == JNE_OK, "open");
+    for (int64_t n : {(int64_t)1, line - 1, line, line + 1, 4 * line}) {
+      check(packed(c, dim, n) == (n > line), "the size rule", dim, n);
+      for (int bps : {4, 6})
+        for (int pack : {1, 0}) {
+          jne_context* d = nullptr;
+          check(jne_open(0, 0, &d) == JNE_OK && jne_set_launch_shape(d, bps, pack) == JNE_OK, "shape");
+          check(packed(d, dim, n) == (pack == 1), "the caller's packing", pack, n);
+          check(fake::mixed.back().a.blocks_per_sm == bps, "the caller's blocks", bps, n);
+          jne_close(d);
+        }
+    }
+    // the tuner: each row times the packing it names; the stored shape leaves the other side of the line to the rule
+    for (int64_t n : {line / 2, 8 * line})
+      for (bool packed_faster : {false, true}) {
+        fake::ms = [&](const fake::MixedLaunch& l) { return (l.a.pack >= 0) == packed_faster ? 1.0f : 2.0f; };
+        jne_tune_entry table[64], best{};
+        int rows = 0;
+        check(jne_autotune(c, dim, 700, 1e-6, 4, n, table, 64, &rows, &best) == JNE_OK, "autotune");
+        for (int r = 0; r < rows; r++)
+          if (table[r].ms >= 0)
+            check(table[r].ms == ((table[r].pack == 1) == packed_faster ? 1.0 : 2.0), "a row's own packing", dim, n);
+        check((best.pack == 1) == packed_faster, "the faster packing is chosen", dim, n);
+        jne_set_chunk(c, JNE_CHUNK_TUNED);
+        check(packed(c, dim, n) == packed_faster, "the choice at the timed size", dim, n);
+        const int64_t other = n > line ? line / 2 : 8 * line;
+        const bool by_rule = packed_faster == (n > line);
+        check(packed(c, dim, other) == (by_rule ? other > line : packed_faster), "the other side of the line", dim, n);
+        jne_set_chunk(c, 0);
+      }
+    jne_close(c);
+  }
+  std::printf("%d failures\n", failures);
+  return failures != 0;
+}

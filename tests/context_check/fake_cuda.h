@@ -6,6 +6,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "../../johansen-null-eigenspectra_gb300/csrc/jne_context.h"
@@ -18,6 +19,8 @@ struct MixedLaunch {
   std::vector<jne_chunk_time> table;  // the chunk table the kernel would read
 };
 
+constexpr int kSms = 3;
+inline std::function<float(const MixedLaunch&)> ms;  // what events around the last mixed launch measure (1 by default)
 inline bool fail_malloc = false, fail_upload = false;
 inline std::vector<MixedLaunch> mixed;
 inline std::vector<std::vector<int4>> entries;  // the entry tables of the FP64 launches on explicit increments
@@ -29,7 +32,7 @@ cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
   *p = nullptr;
   if (fake::fail_malloc) return cudaErrorMemoryAllocation;
-  *p = std::malloc(n ? n : 1);
+  *p = std::calloc(n ? n : 1, 1);
   return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {
@@ -49,19 +52,35 @@ cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) {
   return cudaSuccess;
 }
 cudaError_t cudaMemset(void* p, int v, size_t n) { return cudaMemsetAsync(p, v, n, nullptr); }
+cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
+cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
+cudaError_t cudaGetDeviceCount(int* n) {
+  *n = 1;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) {
+  *v = fake::kSms;
+  return cudaSuccess;
+}
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned int) {
+  *s = nullptr;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned int) { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) {
   *e = nullptr;
   return cudaSuccess;
 }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned int) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
-  *ms = 1.0f;
+  *ms = fake::ms && !fake::mixed.empty() ? fake::ms(fake::mixed.back()) : 1.0f;
   return cudaSuccess;
 }
 }

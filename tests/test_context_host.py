@@ -28,3 +28,7 @@ def _run(tmp_path, name, units=()):
 
 def test_tables_after_a_failed_allocation_or_upload(tmp_path):
     _run(tmp_path, "check_tables")
+
+
+def test_launch_shapes_and_the_tuner(tmp_path):
+    _run(tmp_path, "check_shapes", ["jne_api.cu", "jne_tune.cu"])
