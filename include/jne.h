@@ -98,7 +98,7 @@ typedef struct jne_tune_entry {
   int blocks_per_sm;  /* kernel variant: 4 (128 registers a thread) or 6 (80) */
   int pack;           /* dims <= 4: 1 = two runs per warp, 0 = one */
   double max_rel_err; /* worst max-eig / trace error vs FP64 on the sample (five models), relative to max(value, 1) */
-  double ms;          /* device time of one launch of time_runs runs (model 0); < 0: not timed (over the bound) */
+  double ms;          /* device time of one launch of time_runs runs (model 4, the dearest merge); < 0: not timed (over the bound) */
 } jne_tune_entry;
 
 /* Autotuner of the mixed kernel (no counterpart in the reference, whose only

@@ -57,15 +57,22 @@ struct ModeGuard {
   }
 };
 
-// Device milliseconds of one seeded mixed launch of n runs (model 0) in the
-// context's current mode: a warm-up launch, then the faster of two timed ones.
+// The model the shapes are timed on.  A shape is kept per (dim, class of steps) and
+// serves every model, but the merge carries the moments a model needs: all of them for
+// model 4, the dearest, and none of the sums for model 0 (13 % less time at dim 2, T 1000),
+// on which short chunks would look cheaper than they are.
+constexpr int kTimedModel = 4;
+
+// Device milliseconds of one seeded mixed launch of n runs in the context's
+// current mode: a warm-up launch, then the faster of two timed ones.
 int time_launch(jne_context* c, int dim, int steps, int64_t n, double* d_out, cudaEvent_t e0, cudaEvent_t e1,
                 double* ms) {
   double best = std::numeric_limits<double>::infinity();
   for (int rep = 0; rep < 3; rep++) {
     cudaError_t e = cudaEventRecord(e0, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "tuner event");
-    int rc = jne_eigs_seeded_device(c, 0, dim, steps, JNE_DEFAULT_BASE_SEED, 1, n, JNE_PREC_MIXED, d_out, nullptr);
+    int rc = jne_eigs_seeded_device(c, kTimedModel, dim, steps, JNE_DEFAULT_BASE_SEED, 1, n, JNE_PREC_MIXED, d_out,
+                                    nullptr);
     if (rc) return rc;
     if ((e = cudaEventRecord(e1, c->stream)) != cudaSuccess || (e = cudaEventSynchronize(e1)) != cudaSuccess)
       return cuda_fail(c, e, "tuner event");
@@ -129,7 +136,7 @@ extern "C" int jne_autotune(jne_context* c, int dim, int steps, double max_rel_e
   if (cands.empty()) cands.push_back(32);  // the shortest chunk is the fallback
 
   // 2. the device time of every shape of the admissible chunks
-  const int k0 = jne_eigen_count(0, dim);
+  const int k0 = jne_eigen_count(kTimedModel, dim);
   if ((rc = ensure(c, &c->d_out, &c->out_cap, (size_t)time_runs * k0, "tuner output"))) return rc;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t ce = cudaEventCreate(&e0);

@@ -63,6 +63,23 @@ int main() {
       }
     jne_close(c);
   }
+  {  // the shape serves every model, so the tuner times the one that merges the most moments (every kind: model 4)
+    jne_context* c = nullptr;
+    check(jne_open(0, 0, &c) == JNE_OK, "open");
+    jne_tune_entry table[64], best{};
+    int rows = 0, timed = 0, launches = 0;
+    fake::ms = nullptr;
+    const size_t before = fake::mixed.size();
+    check(jne_autotune(c, 3, 700, 1e-6, 4, 500, table, 64, &rows, &best) == JNE_OK, "autotune");
+    for (int r = 0; r < rows; r++) timed += table[r].ms >= 0;
+    for (size_t i = before; i < fake::mixed.size(); i++)
+      if (fake::mixed[i].a.n_runs == 500) {
+        launches++;
+        check(fake::mixed[i].a.model == 4 && fake::mixed[i].fin_model == 4, "the timed model", fake::mixed[i].a.model);
+      }
+    check(timed > 0 && launches == 3 * timed, "three launches a row", timed, launches);
+    jne_close(c);
+  }
   std::printf("%d failures\n", failures);
   return failures != 0;
 }
