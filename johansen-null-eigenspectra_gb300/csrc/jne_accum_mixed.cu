@@ -21,15 +21,27 @@ __device__ __forceinline__ int request_of(const jne_ragged_req* __restrict__ req
   return lo;
 }
 
+// One unit of a request, its dim's slot table written first where the warp held another dim's.
+template <int DIM>
+__device__ __forceinline__ void ragged_unit(const jne_accum_args& a, int unit, WarpSmem& sm, uint2* slot, int& slot_dim,
+                                            const jne_round_keys& rk, int lane) {
+  if (slot_dim != DIM) {
+    fill_product_slots<DIM, true>(slot, lane, JNE_WARP);
+    __syncwarp();
+    slot_dim = DIM;
+  }
+  accum_unit<DIM, false, false, true>(a, unit, sm, slot, rk, lane);
+}
+
 // batch_done (ceil(total / 32) zeroed counts): every item is also finalized
 // in the launch, batches of 32 consecutive items spanning requests as needed.
 __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
     k_accum_mixed_ragged(const jne_ragged_req* __restrict__ reqs, int n_req, long long total,
                          unsigned long long* __restrict__ counter, unsigned int* __restrict__ batch_done) {
   __shared__ WarpSmem sm_all[kMixWarps];
+  __shared__ uint2 slot_all[kMixWarps][kProductSlots];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  if (lane == 0) sm_all[wib].slot_dim = 0;
-  __syncwarp();
+  int slot_dim = 0;  // the dim this warp's slot table was built for
   // first item by warp, then the next free one from the counter: the warps of a block run the same dim's code
   // (the launch's items are ordered by dim), which fits the instruction cache where several dims' does not
   const unsigned long long nwarps = (unsigned long long)gridDim.x * kMixWarps;
@@ -40,18 +52,18 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 4)
     const int unit = (int)(item - (unsigned long long)reqs[lo].first);
     const jne_round_keys rk = jne_make_round_keys(a.key0, a.key1);
     switch (a.dim) {
-      case 1: accum_unit<1, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 2: accum_unit<2, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 3: accum_unit<3, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 4: accum_unit<4, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 5: accum_unit<5, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 6: accum_unit<6, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 7: accum_unit<7, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 8: accum_unit<8, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 9: accum_unit<9, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 10: accum_unit<10, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      case 11: accum_unit<11, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
-      default: accum_unit<12, false, false, true>(a, unit, sm_all[wib], rk, lane); break;
+      case 1: ragged_unit<1>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 2: ragged_unit<2>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 3: ragged_unit<3>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 4: ragged_unit<4>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 5: ragged_unit<5>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 6: ragged_unit<6>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 7: ragged_unit<7>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 8: ragged_unit<8>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 9: ragged_unit<9>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 10: ragged_unit<10>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      case 11: ragged_unit<11>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
+      default: ragged_unit<12>(a, unit, sm_all[wib], slot_all[wib], slot_dim, rk, lane); break;
     }
     if (batch_done) {
       const long long first = batch_complete(batch_done, (long long)item, total, lane);

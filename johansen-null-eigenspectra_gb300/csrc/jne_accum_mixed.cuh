@@ -405,8 +405,6 @@ struct alignas(16) WarpSmem {
   float2 lt[32];           // Lc * m | chunk increment totals
   float st[32];            // sum b | total z
   float cu[32], cuu[32];   // sum (u - ubar) b | z, sum ((u - ubar)^2 - qbar) b | z
-  uint2 slot[kProductSlots];  // operands of the product slots (see product_slot)
-  int slot_dim;            // dim the slot table was built for
 };
 
 // Which moments of the record a request's model needs beyond the products W W'
@@ -435,6 +433,16 @@ __device__ __forceinline__ uint2 product_slot(int t) {
                     (uint32_t)((o + wb) * kCS + 16 + za) | (uint32_t)(r * NREC + NMWW + 3 * d + v) << 16);
 }
 
+// The product slots' operands of a dim, written by threads `first`, first + stride, ... of those that share the
+// table: a block's warps in the single-request kernels (a table per warp would cost the 6-block variant its sixth
+// block), one warp in the ragged kernel, whose warps may be at different dims.
+template <int DIM, bool PACK>
+__device__ __forceinline__ void fill_product_slots(uint2* slot, int first, int stride) {
+  constexpr int NU = Packing<DIM, PACK>::kRuns, n = NU * (DIM * (DIM + 1) / 2 + DIM * DIM);
+  static_assert(n <= kProductSlots, "slots of a unit fit the table");
+  for (int t = first; t < n; t += stride) slot[t] = product_slot<DIM, NU>(t);
+}
+
 // Lanes that own a walk feature in the merge: lane f < DIM, or (packed) lane
 // 8 r + f of run r.
 template <int DIM, bool PACK>
@@ -444,10 +452,11 @@ __device__ __forceinline__ bool lane_feature_of(int lane) {
 
 // One unit of a request: run `unit`, or (packed dims) runs 2 unit and
 // 2 unit + 1 -- the second only if the request has it: accumulate their moment
-// records into a.mom[slot * a.mom_ld + run].  Executed by a whole warp.
+// records into a.mom[slot * a.mom_ld + run].  Executed by a whole warp; slot is
+// the dim's table (fill_product_slots).
 template <int DIM, bool EXT, bool UNROLL = true, bool PACK = true>
-__device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, WarpSmem& sm, const jne_round_keys& rk,
-                                           int lane) {
+__device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, WarpSmem& sm, const uint2* slot,
+                                           const jne_round_keys& rk, int lane) {
   constexpr int d = DIM;
   constexpr bool PAIR = Packing<DIM, PACK>::kPair;
   constexpr int NU = Packing<DIM, PACK>::kRuns;
@@ -469,11 +478,6 @@ __device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, Wa
   for (int e = lane; e < 16 * kZS; e += 32) {
     const int row = e / kZS;
     if ((PAIR ? (row & 7) : row) >= d) (&zs[0][0])[e] = 0.f;
-  }
-  if (sm.slot_dim != (PAIR ? -d : d)) {  // once per warp, or when a ragged batch changes dim
-    for (int t = lane; t < NU * (NMWW + NNZW); t += 32) sm.slot[t] = product_slot<DIM, NU>(t);
-    __syncwarp();
-    if (lane == 0) sm.slot_dim = PAIR ? -d : d;
   }
   const int kinds = moment_kinds(a.model);
   // G-row coefficients: value = c[0]*b + c[1] + c[2]*u + c[3]*u^2 (packed: the
@@ -636,7 +640,7 @@ __device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, Wa
     // 1208 us, of model 4: 1506 -> 1360; dim 12, T 1000: model 0 6.89 -> 5.86 ms, model 3 7.34 -> 6.39).
     // The products W W' and z W' (a mean product and the centred local part) ...
     for_slots<NU * (NMWW + NNZW), UNROLL>(lane, [&](int t) {
-      const uint2 op = sm.slot[t];
+      const uint2 op = slot[t];
       const int x = op.x & 0xffff, w = op.x >> 16, e = op.y >> 16;
       const float C = (&cm[0][0])[op.y & 0xffff];
       const float2 xv = lt[x], yv = mm[w];
@@ -729,11 +733,14 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, MINB)
     k_accum_mixed(const __grid_constant__ jne_accum_args a, const __grid_constant__ jne_round_keys rk,
                   const __grid_constant__ jne_finalize_args fin) {
   __shared__ WarpSmem sm_all[kMixWarps];
+  __shared__ uint2 slot[kProductSlots];
+  // (1 KB of an SM's 228 goes with every block)
+  static_assert(MINB * (sizeof sm_all + sizeof slot + 1024) <= 228 * 1024, "MINB blocks fit an SM's shared memory");
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nwarps = gridDim.x * kMixWarps;
   const bool fused = fin.out != nullptr && a.batch_done != nullptr;
-  if (lane == 0) sm_all[wib].slot_dim = 0;
-  __syncwarp();
+  fill_product_slots<DIM, PACK>(slot, threadIdx.x, kMixWarps * JNE_WARP);
+  __syncthreads();
   const long long units = jne_units(DIM, a.n_runs, PACK);
   auto finalize_done = [&](long long unit) {
     const long long first = batch_complete(a.batch_done, unit, units, lane);
@@ -742,13 +749,13 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, MINB)
   };
   if (a.next_run == nullptr) {
     for (long long unit = blockIdx.x * kMixWarps + wib; unit < units; unit += nwarps) {
-      accum_unit<DIM, EXT, true, PACK>(a, (int)unit, sm_all[wib], rk, lane);
+      accum_unit<DIM, EXT, true, PACK>(a, (int)unit, sm_all[wib], slot, rk, lane);
       if (fused) finalize_done(unit);
     }
   } else {
     // first unit by warp index, then the next free one from the counter
     for (long long unit = blockIdx.x * kMixWarps + wib; unit < units;) {
-      accum_unit<DIM, EXT, true, PACK>(a, (int)unit, sm_all[wib], rk, lane);
+      accum_unit<DIM, EXT, true, PACK>(a, (int)unit, sm_all[wib], slot, rk, lane);
       if (fused) finalize_done(unit);
       unsigned long long item = 0;
       if (lane == 0) item = atomicAdd(a.next_run, 1ull);
