@@ -10,10 +10,10 @@
 // one such batch.
 #include <algorithm>
 #include <cstring>
-#include <tuple>
 #include <vector>
 
 #include "jne_context.h"
+#include "jne_order.h"
 
 using namespace jne_detail;
 
@@ -111,18 +111,16 @@ std::vector<std::vector<Piece>> plan_launches(const jne_request* reqs, const std
   return out;
 }
 
-// The order in which warps take the units of a launch (results do not depend on
-// it): large dims first, so that the launch ends on short solves (a batch's solve takes
-// 0.5 ms at k = 13, and nothing hides the last one's) and warps of an SM run the same
-// dim's code; within a dim the longest paths first.  The 60-pair plan (128,000 runs)
-// 15.4 -> 12.9 ms; batches of 25 to 60 requests of tens to hundreds of runs 2.0 - 3.3 ->
-// 1.0 - 1.5 ms (longest paths first whatever the dim: 14.3 and 1.7 - 2.7).
-void launch_order(const jne_request* reqs, std::vector<Piece>* pieces) {
-  auto key = [&](const Piece& p) {
+// Puts the pieces of a launch in the order in which warps take them (jne_order.h).
+void order_pieces(const jne_context* c, const jne_request* reqs, std::vector<Piece>* pieces) {
+  std::vector<OrderItem> items;
+  for (const Piece& p : *pieces) {
     const jne_request& r = reqs[p.req];
-    return std::make_tuple(-r.dim, -jne_eigen_count(r.model, r.dim), -r.steps);
-  };
-  std::stable_sort(pieces->begin(), pieces->end(), [&](const Piece& x, const Piece& y) { return key(x) < key(y); });
+    items.push_back({r.dim, jne_eigen_count(r.model, r.dim), r.steps, jne_units(r.dim, p.n)});
+  }
+  std::vector<Piece> out;
+  for (int i : launch_order(items, 16ll * c->sms)) out.push_back((*pieces)[(size_t)i]);  // 4 blocks of 4 warps per SM
+  pieces->swap(out);
 }
 
 // Items of a ragged launch: units, i.e. runs, or pairs of runs for packed dims.
@@ -196,7 +194,7 @@ int jne_detail::run_batch(jne_context* c, const jne_request* reqs, int n_req, do
   cudaError_t e;
   std::vector<std::vector<Piece>> launches = plan_launches(reqs, ragged, cap);
   for (std::vector<Piece>& pieces : launches) {
-    launch_order(reqs, &pieces);
+    order_pieces(c, reqs, &pieces);
     const int b = (int)(c->batch_seq++ & 1);
     // the previous launch that used slot b must be done before its buffers are rewritten
     if (c->fin_pending[b] && (e = cudaEventSynchronize(c->ev_fin[b])) != cudaSuccess)
@@ -434,7 +432,7 @@ int jne_plan_create(jne_context* c, const jne_request* reqs, int n_req, double* 
     pieces.push_back({i, 0, reqs[i].n_runs});
     slots += (size_t)reqs[i].n_runs * jne_record_slots(reqs[i].dim);
   }
-  launch_order(reqs, &pieces);
+  order_pieces(c, reqs, &pieces);
   const size_t ntab = chunks_of(c, reqs, pieces);
   const size_t nbatch = ((size_t)total_units(reqs, pieces) + 31) / 32;
   const unsigned long long bytes = slots * sizeof(double) + pieces.size() * sizeof(jne_ragged_req) +

@@ -32,3 +32,7 @@ def test_tables_after_a_failed_allocation_or_upload(tmp_path):
 
 def test_launch_shapes_and_the_tuner(tmp_path):
     _run(tmp_path, "check_shapes", ["jne_api.cu", "jne_tune.cu"])
+
+
+def test_order_of_a_ragged_launch(tmp_path):
+    _run(tmp_path, "check_order")
