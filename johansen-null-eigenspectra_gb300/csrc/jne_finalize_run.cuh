@@ -64,15 +64,6 @@ struct Ctx {
   }
 };
 
-// 1 / x for normal x: the documented approximation and one third-order Newton
-// step (Householder's method), three FP64 instructions.
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 // Householder reduction of a symmetric n x n matrix to tridiagonal form (Golub &
 // Van Loan, Matrix Computations, Algorithm 8.3.1), given and overwritten as its
 // strict upper triangle (A[i][j], i < j) and diagonal: diagonal -> dg[0..n-1],
@@ -89,7 +80,7 @@ __device__ __forceinline__ void tridiagonalize(double (*A)[JNE_MAX_K], int n, do
     double v[JNE_MAX_K], p[JNE_MAX_K];
     v[k + 1] = x0 - alpha;                        // |x0| + nrm: no cancellation
     for (int i = k + 2; i < n; i++) v[i] = A[k][i];
-    const double tau = reciprocal(fma(nrm, fabs(x0), r2));  // 2 / (v'v)
+    const double tau = 1.0 / fma(nrm, fabs(x0), r2);  // 2 / (v'v)
     for (int i = k + 1; i < n; i++) p[i] = dg[i] * v[i];
     for (int i = k + 1; i < n; i++) {
       const double vi = v[i];

@@ -1,0 +1,27 @@
+"""The finalize near the bottom of the FP64 range: explicit increments so small that the Householder step's squared
+norm is subnormal.  1 / x is then still finite (above 2^-1024) and the eigenvalues those of the unscaled increments
+times c^2.
+
+Tolerance: squares below 2^-1074 are lost, that is rotations among values 2^-537 and smaller, 2^-26 of the matrix's
+2^-511; some fifty such rotations stay within 1e-6."""
+import numpy as np
+import pytest
+
+from conftest import normwise_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits", [-1022.5, -1023.0, -1023.5])
+def test_subnormal_householder_norm(engine, oracle, jne, bits):
+    dB, _ = engine.export_increments(3, 300, 4, 8)
+    ref = oracle.c_eigs_from_increments(0, dB)
+    for run in range(len(dB)):
+        # the pencil of model 0 as the engine forms it: F = the walk, C = E'E with E = S10 L^-T, all unscaled
+        F = np.cumsum(dB[run], axis=0) - dB[run]
+        E = np.linalg.solve(np.linalg.cholesky(F.T @ F), (dB[run].T @ F).T).T
+        C = E.T @ E
+        r2 = C[0, 1] ** 2 + C[0, 2] ** 2
+        c = 2.0 ** ((bits - np.log2(np.sqrt(r2) * abs(C[0, 1]) + r2)) / 4)  # C scales with c^2, its squares with c^4
+        got = engine.eigs_from_increments(0, dB[run:run + 1] * c, precision=jne.PREC_FP64)
+        assert normwise_err(got / c / c, ref[run:run + 1]) < 1e-6, run
