@@ -20,7 +20,8 @@
 // Accumulator range.  G_s holds integers below 2^24 exactly:
 //   * d0 is bounded by ending the chunk (for any reason a chunk may end: the
 //     merge takes any length) once the walk has passed jne_digit_limit, 6.8
-//     standard deviations of a full chunk;
+//     standard deviations of a full chunk (a packed pair of which one run does so is
+//     computed run by run, digit_pair_apart);
 //   * the squares on the diagonal are the only sums that grow with the chunk's
 //     length rather than its root: their expectation, (1024^2 - 1) / 12 a step
 //     for uniform digits, is taken out of the accumulator tile by tile and put
@@ -312,9 +313,11 @@ __device__ __forceinline__ void digit_tile(const float (*zs)[kZS], const uint32_
   }
 }
 
-// One unit of a request (see accum_unit): its moment records into a.mom.
+// One unit of a request (see accum_unit): its moment records into a.mom.  False, and
+// nothing written, for a pair of which one run's walk has passed the limit: where chunks
+// end shows in a run's last bits, which must not depend on the run it is paired with.
 template <int DIM, bool PACK>
-__device__ __forceinline__ void digit_unit(const jne_accum_args& a, int unit, DigSmem& sm, const jne_round_keys& rk,
+__device__ __forceinline__ bool digit_unit(const jne_accum_args& a, int unit, DigSmem& sm, const jne_round_keys& rk,
                                            int lane) {
   constexpr int d = DIM;
   constexpr bool PAIR = Packing<DIM, PACK>::kPair;
@@ -367,7 +370,7 @@ __device__ __forceinline__ void digit_unit(const jne_accum_args& a, int unit, Di
 #pragma unroll
         for (int r = 0; r < 4; r++) acc[n][s][r] = 0.f;
     long long carA = 0, carB = 0;
-    int t0 = c0;
+    int t0 = c0, over = 0;
     for (;;) {
       const int i = t0 + lane;
       const bool valid = i < T;
@@ -403,10 +406,14 @@ __device__ __forceinline__ void digit_unit(const jne_accum_args& a, int unit, Di
                                      diag1, acc);
       __syncwarp();
       t0 += 32;
+      if (PAIR) over = max(over, max(abs((int)(carA >> 32)), abs((int)(carB >> 32))));
       if (t0 >= T || t0 - c0 >= L) break;
-      const int hA = abs((int)(carA >> 32)), hB = BLOCK1 && (PAIR || g < 4) ? abs((int)(carB >> 32)) : 0;
-      if (__any_sync(0xffffffffu, max(hA, hB) > limit)) break;
+      if (!PAIR) {
+        const int hA = abs((int)(carA >> 32)), hB = BLOCK1 && g < 4 ? abs((int)(carB >> 32)) : 0;
+        if (__any_sync(0xffffffffu, max(hA, hB) > limit)) break;
+      }
     }
+    if (PAIR && __any_sync(0xffffffffu, over > limit)) return false;
     const int Lc = min(t0, T) - c0;
     const int ntile = (t0 - c0) >> 5;
     // the squares of d3 left out with G_6 have a mean too, (1024^2 - 1) / 12 for every step but the chunk's first
@@ -518,6 +525,18 @@ __device__ __forceinline__ void digit_unit(const jne_accum_args& a, int unit, Di
     if (r < nrun) a.mom[(size_t)e * ld + run0 + r] = sm.rec[t];
   }
   __syncwarp();
+  return true;
+}
+
+// The runs of a pair by themselves, as the unpacked kernel computes them (a walk passes the limit with
+// probability 2e-11 per feature and chunk).  A call, and a check once a chunk, so that neither its registers
+// nor its code touch the packed kernel's loop: ending the pair's chunk there and starting over with one run's
+// chunks cost 3 - 4 % at dims 1 to 4, T 1000; this form -0.5 % at dims 1, 2 and 4, +2 % at dim 3 (T 10^4: -7 %).
+template <int DIM>
+__device__ __noinline__ void digit_pair_apart(const jne_accum_args& a, int unit, DigSmem& sm, const jne_round_keys& rk,
+                                              int lane) {
+  __syncwarp();
+  for (int run = 2 * unit; run < min(2 * unit + 2, a.n_runs); run++) digit_unit<DIM, false>(a, run, sm, rk, lane);
 }
 
 template <int DIM, bool PACK>
@@ -531,7 +550,9 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 3)
   const long long units = jne_units(DIM, a.n_runs, PACK);
   // first unit by warp index, then the next free one from the counter
   for (long long unit = blockIdx.x * kMixWarps + wib; unit < units;) {
-    digit_unit<DIM, PACK>(a, (int)unit, sm_all[wib], rk, lane);
+    const bool written = digit_unit<DIM, PACK>(a, (int)unit, sm_all[wib], rk, lane);
+    if constexpr (Packing<DIM, PACK>::kPair)
+      if (!written) digit_pair_apart<DIM>(a, (int)unit, sm_all[wib], rk, lane);
     if (fused) {
       const long long first = batch_complete(a.batch_done, unit, units, lane);
       if (first >= 0) finalize_batch(fin, first, PACK, lane);
