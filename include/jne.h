@@ -174,7 +174,7 @@ int jne_eigs_seeded_models(jne_context* ctx, const int* models, int n_models, in
  * jne_noalloc_last_error (per thread). */
 #define JNE_NOALLOC_MAX_RUNS 2048
 #define JNE_NOALLOC_MAX_CHUNKS 4096
-#define JNE_NOALLOC_SCRATCH_BYTES 4956672
+#define JNE_NOALLOC_SCRATCH_BYTES 4948480
 int jne_eigs_seeded_noalloc(int device, int model, int dim, int steps, uint64_t base_seed, uint32_t seed_first,
                             int n_runs, int precision, double* out_device, void* stream);
 const char* jne_noalloc_last_error(void);

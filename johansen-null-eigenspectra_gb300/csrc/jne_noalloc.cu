@@ -28,12 +28,11 @@ constexpr size_t round_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign;
 constexpr int kRecordMax = JNE_MAX_DIM * (JNE_MAX_DIM + 1) / 2 + 6 * JNE_MAX_DIM + JNE_MAX_DIM * JNE_MAX_DIM;
 constexpr size_t kMomBytes = round_up(sizeof(double) * (size_t)JNE_NOALLOC_MAX_RUNS * kRecordMax);
 constexpr size_t kChunkBytes = round_up(sizeof(jne_chunk_time) * (size_t)JNE_NOALLOC_MAX_CHUNKS);
-constexpr size_t kReservedBytes = 8192;  // keeps the scratch size jne.h states
-// status word (offset 0) and the mixed kernel's work counter (offset 8)
+// status word (offset 0) and the kernels' work counter (offset 8)
 constexpr size_t kWordsBytes = kAlign;
 // completion counts of the fused finalize, one per 32 runs
 constexpr size_t kBatchBytes = round_up(sizeof(unsigned int) * ((JNE_NOALLOC_MAX_RUNS + 31) / 32));
-constexpr size_t kScratchBytes = kMomBytes + kChunkBytes + kReservedBytes + kWordsBytes + kBatchBytes;
+constexpr size_t kScratchBytes = kMomBytes + kChunkBytes + kWordsBytes + kBatchBytes;
 static_assert(kScratchBytes == JNE_NOALLOC_SCRATCH_BYTES, "scratch size stated in jne.h");
 
 static __device__ __align__(256) unsigned char jne_noalloc_scratch[kScratchBytes];
@@ -97,7 +96,7 @@ extern "C" int jne_eigs_seeded_noalloc(int device, int model, int dim, int steps
   const int sms = g_sms[device];
   double* mom = reinterpret_cast<double*>(base);
   jne_chunk_time* ctab = reinterpret_cast<jne_chunk_time*>(base + kMomBytes);
-  unsigned char* words = base + kMomBytes + kChunkBytes + kReservedBytes;
+  unsigned char* words = base + kMomBytes + kChunkBytes;
   unsigned int* status = reinterpret_cast<unsigned int*>(words);
   unsigned long long* next_run = reinterpret_cast<unsigned long long*>(words + 8);
   unsigned int* batch_done = reinterpret_cast<unsigned int*>(words + kWordsBytes);
