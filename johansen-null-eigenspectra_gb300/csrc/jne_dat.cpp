@@ -726,6 +726,8 @@ namespace {
 // places, given that v[lo..hi) holds the values of those places.
 void select_ranks(double* v, int64_t lo, int64_t hi, const int64_t* ranks, size_t a, size_t b) {
   if (a >= b) return;
+  // values that are all the same are in place (the look ends at the first that differs)
+  if (std::all_of(v + lo, v + hi, [&](double x) { return x == v[lo]; })) return;
   const size_t m = a + (b - a) / 2;
   std::nth_element(v + lo, v + ranks[m], v + hi);
   select_ranks(v, lo, ranks[m], ranks, a, m);
@@ -794,16 +796,22 @@ int jne_percentiles(const double* eigs, int64_t n, int k, int stat, const double
   // the reference's sort (partial_cmp().unwrap(), simulation_analyzers.rs:60) panics on NaN
   if (nans) return dat_fail(JNE_ERR_NUMERIC, std::to_string(nans) + " runs have a NaN aggregate (unordered)");
   // only the order statistics next to the wanted ranks: each selected within the range its neighbours left, halving
-  // the list of ranks (200,000 x 5 values, 7 percentiles, the sums included: 3.6 ms, sorted 10.6)
-  std::vector<int64_t> ranks;
-  for (int i = 0; i < np && n > 0; i++) {
-    const double rank = ps[i] * (double)(n - 1);
-    ranks.push_back((int64_t)std::floor(rank));
-    ranks.push_back((int64_t)std::ceil(rank));
+  // the list of ranks (200,000 x 5 values, 7 percentiles, the sums included: 3.6 ms, sorted 10.6).  Many ranks of
+  // few values are sorted: up to 32 values a percentile (1000 values, 101 percentiles: selected 46 us, sorted 24;
+  // 30,000 values 1.09 ms, 1.45).
+  if (n < 32 * (int64_t)np) {
+    std::sort(v.begin(), v.end());
+  } else {
+    std::vector<int64_t> ranks;
+    for (int i = 0; i < np; i++) {
+      const double rank = ps[i] * (double)(n - 1);
+      ranks.push_back((int64_t)std::floor(rank));
+      ranks.push_back((int64_t)std::ceil(rank));
+    }
+    std::sort(ranks.begin(), ranks.end());
+    ranks.erase(std::unique(ranks.begin(), ranks.end()), ranks.end());
+    select_ranks(v.data(), 0, n, ranks.data(), 0, ranks.size());
   }
-  std::sort(ranks.begin(), ranks.end());
-  ranks.erase(std::unique(ranks.begin(), ranks.end()), ranks.end());
-  select_ranks(v.data(), 0, n, ranks.data(), 0, ranks.size());
   for (int i = 0; i < np; i++) {  // simulation_analyzers.rs:4-18
     if (n == 0) {
       out[i] = NAN;
