@@ -6,15 +6,16 @@
 // all aggregates; only the two order statistics around each rank p (n - 1) are
 // needed, so they are found by a most-significant-digit select on
 // order-preserving 64-bit keys less their minimum: a first histogram of up to
-// 2048 bins over the keys' actual range, then 7 bits a pass for each wanted rank's
-// bin, until a bin holds at most 64 keys, which the next pass lists.  The selected
-// keys are exact aggregate values, and the interpolation runs on the host with the
-// reference's arithmetic, so the result is bit-identical to a full sort.
+// 2048 bins over the keys' actual range, then 128 bins a pass over each wanted rank's
+// bin (where many keys share it, over the range that the last pass found them in), until
+// that range is one key (tied values) or a bin holds at most 64 keys, which the next pass
+// lists.  The selected keys are exact aggregate values, and the interpolation runs on the
+// host with the reference's arithmetic, so the result is bit-identical to a full sort.
 //
 // What bounds it: for 10^6 runs of 12 values the 96 MB read (15 us at the copy
 // bandwidth) and, for the sums, the FP64 additions (19 us); the passes read 8 MB of
-// keys from L2, and all but the first skip a key by one bit of a map of the selected
-// first bins.  Each pass's last block picks the bins and clears the counters, so a
+// keys from L2, and all but the first take a key to its ranks (mostly none) by a table of
+// the first bins.  Each pass's last block picks the bins and clears the counters, so a
 // pass is one launch; three resolve distinct values, and the host starts more only
 // when they did not.  10^6 x 12, seven percentiles: 444 us before (eight passes of
 // three launches, each comparing every key with every rank's prefix), 130 now, of
@@ -54,16 +55,19 @@ struct QHead {
   unsigned long long neg_min, max;  // ~smallest and largest key (both start at 0)
   unsigned long long todo;          // ranks of the group still open (bit per rank)
 };
-constexpr int kHeadWords = sizeof(QHead) / 8 + 1;  // and the shifts
+constexpr int kHeadWords = sizeof(QHead) / 8 + 1;  // and the shift
+constexpr int kRankWords = 6;                      // arrays per rank
 
 // The scratch after the keys.
 struct QLayout {
   QHead* head;
-  unsigned int* shifts;        // [0] bits below the first digit, [1] below the current one
-  unsigned long long* prefix;  // per rank: (key - min) >> shifts[1]; the key itself once closed
+  unsigned int* shift;         // bits below the first digit
+  unsigned long long* lo;      // per rank: its bin's first key; the rank's own key once closed
+  unsigned long long* hi;      // per rank: its bin's last key
   unsigned long long* rank;    // per rank: rank within its bin
   unsigned long long* count;   // per rank: keys in its bin, twice (high and low half)
-  unsigned int* map;           // first-pass bins selected by some rank (a bit each)
+  unsigned long long* nmin;    // per rank: ~smallest and largest key found in its bin (both start at 0)
+  unsigned long long* max;
   unsigned int* hist;          // bins of the current pass (kSub per rank after the first), or a small bin's keys
 };
 
@@ -226,10 +230,12 @@ __global__ void __launch_bounds__(kPassThreads) k_select_first(const unsigned lo
     unsigned long long r = ranks.r[w], c;
     const int b = pick(sh, bins, r, c);
     if ((threadIdx.x & 31) == 0) {
-      q.prefix[w] = (unsigned long long)b + (s1 == 0 ? kmin : 0ull);
+      const unsigned long long at = (unsigned long long)b << s1;
+      q.lo[w] = kmin + at;
+      q.hi[w] = kmin + min(range, at + ((1ull << s1) - 1ull));
       q.rank[w] = r;
       q.count[w] = c << 32 | c;
-      atomicOr(&q.map[b >> 5], 1u << (b & 31));
+      q.nmin[w] = q.max[w] = 0ull;
     }
   }
   __syncthreads();
@@ -237,83 +243,123 @@ __global__ void __launch_bounds__(kPassThreads) k_select_first(const unsigned lo
   if (threadIdx.x == 0) {
     q.head->ticket = 0;
     q.head->todo = s1 == 0 ? 0ull : (1ull << nr) - 1ull;  // without lower bits a bin is one key
-    q.shifts[0] = q.shifts[1] = (unsigned int)s1;
+    *q.shift = (unsigned int)s1;
   }
 }
 
-// A later pass: the next bits of the keys in each open rank's bin; a bin of at
-// most kList keys is listed instead (in its counters' place), and the rank's key
-// taken from the list.
+// A later pass: a histogram over each open rank's bin; a bin of at most kList keys is
+// listed instead (in its counters' place), and the rank's key taken from the list.  Ranks
+// of one bin (neighbours, as a percentile's two mostly are) share the first one's.  In a
+// bin of sixteen times its share of the keys, ties or a cluster are likely: such bins are
+// counted per block in shared memory (tied keys would meet at one global counter) and
+// the range that their keys lie in is found too (10^6 values of three kinds, seven
+// percentiles: 690 us before, 92 now).
 __global__ void __launch_bounds__(kPassThreads) k_select_next(const unsigned long long* __restrict__ keys, long long n,
                                                              int bins, int nr, const __grid_constant__ QLayout q) {
-  __shared__ unsigned int map[kFirstMax / 32];
-  __shared__ unsigned long long pf[kGroup], left;
-  __shared__ bool small[kGroup];
+  __shared__ __align__(4) unsigned short ranks_of[kFirstMax];  // of each first bin, a bit each
+  __shared__ unsigned long long lo[kGroup], span[kGroup], found_min[kGroup], found_max[kGroup], left;
+  __shared__ int shift[kGroup], first_of[kGroup];
+  __shared__ bool small[kGroup], dense[kGroup];
   __shared__ __align__(8) unsigned int sh[kGroup * kSub];
   const unsigned long long todo = q.head->todo;
   if (todo == 0) return;  // the same for every block: an earlier launch wrote it
   const unsigned long long kmin = ~q.head->neg_min;
-  const int s1 = (int)q.shifts[0], s = (int)q.shifts[1], d = min(s, kSubBits);
-  if (threadIdx.x < bins / 32) map[threadIdx.x] = q.map[threadIdx.x];
+  const int s1 = (int)*q.shift;
+  for (int i = threadIdx.x; i < bins / 2; i += kPassThreads) reinterpret_cast<unsigned int*>(ranks_of)[i] = 0;
   if (threadIdx.x < nr) {
-    pf[threadIdx.x] = q.prefix[threadIdx.x];
-    small[threadIdx.x] = (q.count[threadIdx.x] >> 32) <= kList;
+    const int g = threadIdx.x;
+    lo[g] = q.lo[g];
+    span[g] = q.hi[g] - lo[g];
+    shift[g] = max(0, 64 - __clzll((long long)span[g]) - kSubBits);
+    small[g] = (q.count[g] >> 32) <= kList;
+    dense[g] = !small[g] && (q.count[g] >> 32) > 16ull * (unsigned long long)n / (unsigned int)bins;
+    found_min[g] = ~0ull;
+    found_max[g] = 0ull;
+    int f = 0;  // the first open rank of the same bin (ranks' bins do not overlap otherwise)
+    while (f < g && !((todo >> f & 1ull) && q.lo[f] == lo[g] && q.hi[f] == q.hi[g])) f++;
+    first_of[g] = f;
   }
+  for (int i = threadIdx.x; i < nr * kSub; i += kPassThreads) sh[i] = 0;
   if (threadIdx.x == 0) left = todo;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int g = 0; g < nr; g++)
+      if ((todo >> g & 1ull) && first_of[g] == g) ranks_of[(lo[g] - kmin) >> s1] |= (unsigned short)(1u << g);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   for_keys(keys, n, [&](unsigned long long key, bool valid) {
-    const unsigned long long v = valid ? key - kmin : 0ull;
-    const unsigned int b = (unsigned int)(v >> s1);
-    const bool hit = valid && (map[b >> 5] >> (b & 31) & 1u);
-    if (!__any_sync(0xffffffffu, hit)) return;
-    const unsigned long long hi = v >> s;
-    for (int g = 0; g < nr; g++) {
-      const bool m = hit && (todo >> g & 1ull) && hi == pf[g];
+    const unsigned int mine = valid ? ranks_of[(key - kmin) >> s1] : 0u;
+    if (!__any_sync(0xffffffffu, mine != 0)) return;
+    for (unsigned int some = __reduce_or_sync(0xffffffffu, mine); some; some &= some - 1u) {
+      const int g = __ffs(some) - 1;
+      const unsigned long long at = key - lo[g];
+      const bool m = (mine >> g & 1u) && at <= span[g];
       if (!__any_sync(0xffffffffu, m)) continue;
       if (small[g]) {
         if (m) {
-          const unsigned int at = atomicAdd(reinterpret_cast<unsigned int*>(&q.count[g]), ~0u) - 1u;
-          reinterpret_cast<unsigned long long*>(q.hist + g * kSub)[at] = v + kmin;
+          const unsigned int place = atomicAdd(reinterpret_cast<unsigned int*>(&q.count[g]), ~0u) - 1u;
+          reinterpret_cast<unsigned long long*>(q.hist + g * kSub)[place] = key;
         }
       } else {
-        const unsigned int bin = (unsigned int)(v >> (s - d)) & ((1u << d) - 1u);
+        const unsigned int bin = (unsigned int)(at >> shift[g]);
         const unsigned int peers = __match_any_sync(0xffffffffu, m ? bin : 0x1000u + lane);
-        if (m && lane == __ffs(peers) - 1) atomicAdd(&q.hist[g * kSub + bin], (unsigned int)__popc(peers));
+        if (m && lane == __ffs(peers) - 1)
+          atomicAdd(dense[g] ? &sh[g * kSub + bin] : &q.hist[g * kSub + bin], (unsigned int)__popc(peers));
+        if (m && dense[g]) {  // (a stale look only makes the atomic superfluous)
+          if (key < *(volatile unsigned long long*)&found_min[g]) atomicMin(&found_min[g], key);
+          if (key > *(volatile unsigned long long*)&found_max[g]) atomicMax(&found_max[g], key);
+        }
       }
     }
   });
+  __syncthreads();
+  for (int i = threadIdx.x; i < nr * kSub; i += kPassThreads)
+    if (dense[i / kSub] && sh[i]) atomicAdd(&q.hist[i], sh[i]);
+  if (threadIdx.x < nr && found_min[threadIdx.x] <= found_max[threadIdx.x]) {
+    atomicMax(&q.nmin[threadIdx.x], ~found_min[threadIdx.x]);
+    atomicMax(&q.max[threadIdx.x], found_max[threadIdx.x]);
+  }
   if (!last_block(&q.head->ticket)) return;
   for (int i = threadIdx.x; i < nr * kSub; i += kPassThreads) {
     sh[i] = __ldcg(&q.hist[i]);
     q.hist[i] = 0;
   }
+  // what the bin's first rank counted, ahead of that rank's warp writing its next bin
+  const int w = threadIdx.x >> 5, f = w < nr ? first_of[w] : 0;
+  const unsigned long long least = ~__ldcg(&q.nmin[f]), most = __ldcg(&q.max[f]);
+  const int c_list = (int)(__ldcg(&q.count[f]) >> 32);
   __syncthreads();
-  const int w = threadIdx.x >> 5;
   if (w < nr && (todo >> w & 1ull)) {
     unsigned long long r = q.rank[w];
     if (small[w]) {  // the key with r others before it (equal keys in list order)
-      const unsigned long long* list = reinterpret_cast<const unsigned long long*>(sh + w * kSub);
-      const int c = (int)(__ldcg(&q.count[w]) >> 32);
-      for (int i = lane; i < c; i += 32) {
+      const unsigned long long* list = reinterpret_cast<const unsigned long long*>(sh + f * kSub);
+      for (int i = lane; i < c_list; i += 32) {
         const unsigned long long x = list[i];
         unsigned long long before = 0;
-        for (int j = 0; j < c; j++) {
+        for (int j = 0; j < c_list; j++) {
           const unsigned long long y = list[j];
           before += y < x || (y == x && j < i);
         }
-        if (before == r) q.prefix[w] = x;
+        if (before == r) q.lo[w] = x;
       }
       if (lane == 0) atomicAnd(&left, ~(1ull << w));
     } else {
       unsigned long long c;
-      const int b = pick(sh + w * kSub, kSub, r, c);
+      const int b = pick(sh + f * kSub, kSub, r, c);
       if (lane == 0) {
-        const unsigned long long p = (pf[w] << d) | (unsigned long long)b;
-        q.prefix[w] = s == d ? p + kmin : p;
+        // the picked bin, as far as keys were found in it
+        const unsigned long long at = (unsigned long long)b << shift[w];
+        unsigned long long first = lo[w] + at, last = lo[w] + min(span[w], at + ((1ull << shift[w]) - 1ull));
+        if (dense[w]) {
+          first = max(first, least);
+          last = min(last, most);
+        }
+        q.lo[w] = first;
+        q.hi[w] = last;
         q.rank[w] = r;
         q.count[w] = c << 32 | c;
-        if (s == d) atomicAnd(&left, ~(1ull << w));
+        q.nmin[w] = q.max[w] = 0ull;
+        if (first == last) atomicAnd(&left, ~(1ull << w));
       }
     }
   }
@@ -321,7 +367,6 @@ __global__ void __launch_bounds__(kPassThreads) k_select_next(const unsigned lon
   if (threadIdx.x == 0) {
     q.head->ticket = 0;
     q.head->todo = left;
-    q.shifts[1] = (unsigned int)(s - d);
   }
 }
 
@@ -353,20 +398,22 @@ extern "C" int jne_percentiles_device(jne_context* c, const double* eigs_device,
   std::sort(ranks.begin(), ranks.end());
   ranks.erase(std::unique(ranks.begin(), ranks.end()), ranks.end());
   const int nr = (int)ranks.size();
-  // scratch: keys | head, shifts | per rank of a group: prefix, rank, count | map of first bins | histogram
+  // scratch: keys | head, shift | the arrays per rank of a group | histogram
   const int ngmax = std::min(nr, kGroup), bins = first_bins(ngmax);
-  const size_t hist_words = (size_t)std::max(bins, ngmax * kSub) / 2, map_words = (size_t)bins / 64;
-  const size_t words = (size_t)n + kHeadWords + 3 * (size_t)ngmax + map_words + hist_words;
+  const size_t hist_words = (size_t)std::max(bins, ngmax * kSub) / 2;
+  const size_t words = (size_t)n + kHeadWords + kRankWords * (size_t)ngmax + hist_words;
   if ((rc = ensure(c, &c->d_qscratch, &c->qscratch_cap, words, "percentile scratch"))) return rc;
   unsigned long long* keys = c->d_qscratch;
   QLayout q;
   q.head = reinterpret_cast<QHead*>(keys + n);
-  q.shifts = reinterpret_cast<unsigned int*>(keys + n + kHeadWords - 1);
-  q.prefix = keys + n + kHeadWords;
-  q.rank = q.prefix + ngmax;
+  q.shift = reinterpret_cast<unsigned int*>(keys + n + kHeadWords - 1);
+  q.lo = keys + n + kHeadWords;  // read back with the head
+  q.hi = q.lo + ngmax;
+  q.rank = q.hi + ngmax;
   q.count = q.rank + ngmax;
-  q.map = reinterpret_cast<unsigned int*>(q.count + ngmax);
-  q.hist = q.map + 2 * map_words;
+  q.nmin = q.count + ngmax;
+  q.max = q.nmin + ngmax;
+  q.hist = reinterpret_cast<unsigned int*>(q.max + ngmax);
   cudaStream_t st = c->stream;
   cudaError_t e = cudaMemsetAsync(keys + n, 0, sizeof(unsigned long long) * (words - (size_t)n), st);
   if (e != cudaSuccess) return cuda_fail(c, e, "percentile setup");
@@ -385,8 +432,6 @@ extern "C" int jne_percentiles_device(jne_context* c, const double* eigs_device,
     const int ng = std::min(kGroup, nr - g0);
     QRanks gr{};
     for (int g = 0; g < ng; g++) gr.r[g] = ranks[(size_t)(g0 + g)];
-    if (g0 > 0 && (e = cudaMemsetAsync(q.map, 0, sizeof(unsigned long long) * map_words, st)) != cudaSuccess)
-      return cuda_fail(c, e, "percentile setup");
     k_select_first<<<grid_pass, kPassThreads, 0, st>>>(keys, n, bins, ng, gr, q);
     unsigned long long todo = 1;
     // at most 57 bits below the first digit, 7 a pass, and one more for a rank alone in its bin
