@@ -87,7 +87,8 @@ int jne_set_chunk(jne_context* ctx, int chunk);
  * blocks_per_sm 4 (the default, also as 0; 128 registers a thread) or 6 (80),
  * and for dims up to 4 pack = 1 (two runs per warp) or 0 (one) whatever the
  * request's size.  A context on which this was never called packs requests of
- * more than 16 runs per SM only: fewer runs each have a warp of their own.
+ * more than 16 runs per SM only (12 where steps > 1000 dim^2): fewer runs each
+ * have a warp of their own.
  * Speed only: every variant gives the same bits.  No counterpart in the
  * reference. */
 int jne_set_launch_shape(jne_context* ctx, int blocks_per_sm, int pack);

@@ -270,7 +270,7 @@ class Engine:
     def set_launch_shape(self, blocks_per_sm: int = 4, pack: int = 1) -> None:
         """The mixed kernel variant outside CHUNK_TUNED mode: 4 or 6 blocks per SM; for dims <= 4 two runs
         per warp (pack=1) or one (pack=0), whatever the request's size (an engine on which this was never called
-        packs past 16 runs per SM).  Speed only: the same bits."""
+        packs past 16 runs per SM, or 12 where steps > 1000 dim^2).  Speed only: the same bits."""
         self._check(self._L.jne_set_launch_shape(self._h, blocks_per_sm, pack))
 
     def autotune(self, dim: int, steps: int, max_rel_err: float = 1e-6, sample_runs: int = 2000,

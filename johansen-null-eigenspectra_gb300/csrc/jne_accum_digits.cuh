@@ -567,8 +567,7 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, 3)
 template <int DIM>
 cudaError_t launch_digits_dim(const jne_accum_args& a, const jne_finalize_args& fin, int sms, cudaStream_t st) {
   const int threads = kMixWarps * JNE_WARP;
-  // small dims pack two runs per warp once every run can no longer have a warp of its own (3 blocks of 4 per SM)
-  const bool pack = DIM <= JNE_PACK_MAX_DIM && a.n_runs > 12 * sms;
+  const bool pack = DIM <= JNE_PACK_MAX_DIM && jne_digits_pack(DIM, a.steps, a.n_runs, sms);
   auto k = pack ? k_accum_digits<DIM, (DIM <= JNE_PACK_MAX_DIM)> : k_accum_digits<DIM, false>;
   k<<<resident_grid(k, threads, 0, sms, jne_units(DIM, a.n_runs, pack), kMixWarps), threads, 0, st>>>(
       a, jne_make_round_keys(a.key0, a.key1), fin);

@@ -3,8 +3,9 @@
 //
 // Same contract as the plain FP64 kernel (it replaces rng_matrix.rs:57-141,
 // johansen_statistics.rs:102-197 and the two sum_of_outer_products calls of
-// johansen_statistics.rs:32-33) and writes the same FP64 moment record, always
-// the full record, so one pass serves every model.
+// johansen_statistics.rs:32-33) and writes the same FP64 moment record: the moments
+// the request's model needs, the other sums zero, or every one in a pass that serves
+// several models.
 //
 // Time is cut into chunks of `chunk` steps (multiple of 32).  Inside a chunk
 // the walk is taken relative to its value Wc at the chunk start (origin
@@ -691,7 +692,7 @@ __device__ __forceinline__ void accum_unit(const jne_accum_args& a, int unit, Wa
 
 // Fused finalize.  Units (runs, or packed pairs of runs) are counted per batch
 // of 32 consecutive items; the warp that accumulates the last unit of a batch
-// finalizes the whole batch, one unit per lane, in FP64 -- a pipe the accumulation leaves idle, so the
+// finalizes the whole batch, one run per lane, in FP64 -- a pipe the accumulation leaves idle, so the
 // finalize runs in the shadow of the other warps' accumulation instead of in a
 // second kernel after it.  Every batch is full except the very last, and a
 // lane's record reads are contiguous with its neighbours'.  Ordering: the

@@ -371,7 +371,7 @@ inline int accumulate(jne_context* c, int model, int dim, int steps, uint32_t ke
     a.chunk_tab = c->d_ctab;
     const jne_shape shape = shape_for(c, dim, steps);
     a.blocks_per_sm = d_ext ? 4 : shape.blocks_per_sm;
-    const bool pack = shape.pack < 0 ? jne_pack_by_default(n, c->sms) : shape.pack != 0;
+    const bool pack = shape.pack < 0 ? jne_pack_by_default(dim, steps, n, c->sms) : shape.pack != 0;
     a.pack = d_ext || pack ? 0 : -1;
   }
   // warps take runs from a counter, so warps that start late or finalize take fewer

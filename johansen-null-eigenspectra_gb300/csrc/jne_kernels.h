@@ -21,8 +21,24 @@ __host__ __device__ __forceinline__ long long jne_units(int dim, long long n_run
 // Whether the mixed single-request kernel packs when nobody chose: one run per warp
 // while every run has a warp of its own (4 blocks of 4 warps per SM); packed, half the
 // warps would do twice the work (608 runs: dim 2, T 1000 106 -> 77 us, dim 4 210 -> 129,
-// dim 3, T 10^4 284 -> 199; equal at 2,432 runs, and 1.3x the other way at 4,864).
-inline bool jne_pack_by_default(long long n_runs, int sms) { return n_runs > 16ll * sms; }
+// dim 3, T 10^4 284 -> 199).  From 12 runs per SM on (a fourth warp on every scheduler) long
+// paths of the smallest dims are packed too, whose two runs cost little more than one:
+// time unpacked over packed at 2,000 runs, T 1000, 5000, 10^4: dim 1 0.99, 1.17, 1.24; dim 2
+// 0.83, 1.01, 1.11; dim 3 0.74, 0.92, 1.03; dim 4 0.67, 0.84, 0.95.
+inline bool jne_pack_by_default(int dim, int steps, long long n_runs, int sms) {
+  return n_runs > ((long long)steps > 1000ll * dim * dim ? 12ll : 16ll) * sms;
+}
+
+// The same for the FP64 digits (3 blocks of 4 warps per SM).  A batch of packed pairs is
+// solved in two rounds, which on short paths is most of the time until the solves fill the
+// GPU: time unpacked over packed at dim 4, T 33 and 2,000, 9,728, 20,000 runs 0.61, 0.72,
+// 0.84; T 400 0.73, 0.95, 1.06; T 1000 and 2,000, 3,648 runs 0.80, 0.92; dim 3, T 200 and
+// 2,000, 20,000 runs 0.75, 1.03; dim 2, T 100 0.75, 1.06, T 400 and 3,040 runs 1.11; dim 1 0.98
+// and more past 1,824 runs.
+inline bool jne_digits_pack(int dim, int steps, long long n_runs, int sms) {
+  const long long line = 3000ll * dim * (dim - 1) / steps;
+  return n_runs > (line < 12 ? 12 : line > 80 ? 80 : line) * sms;
+}
 
 // Argument block of the finalize kernel.
 struct jne_finalize_args {

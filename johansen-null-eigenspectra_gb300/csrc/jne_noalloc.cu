@@ -136,7 +136,7 @@ extern "C" int jne_eigs_seeded_noalloc(int device, int model, int dim, int steps
       a.chunk_tab = ctab;
       a.next_run = next_run;
       a.batch_done = batch_done;
-      a.pack = jne_pack_by_default(n_runs, sms) ? 0 : -1;
+      a.pack = jne_pack_by_default(dim, steps, n_runs, sms) ? 0 : -1;
       if (e == cudaSuccess) e = jne_launch_accum_mixed(a, &f, sms, st);  // accumulation + fused finalize
     } else {
       a.next_run = next_run;

@@ -169,7 +169,7 @@ extern "C" int jne_autotune(jne_context* c, int dim, int steps, double max_rel_e
   if (rc) return rc;
   // where the size rule would have chosen the same packing, it goes on choosing: a pick at time_runs runs says
   // nothing about requests on the other side of its line
-  const bool as_rule = (best.pack != 0) == jne_pack_by_default(time_runs, c->sms);
+  const bool as_rule = (best.pack != 0) == jne_pack_by_default(dim, tb, time_runs, c->sms);
   c->tuned[{dim, b}] = jne_shape{best.chunk, best.blocks_per_sm, as_rule ? -1 : best.pack};
   if (chosen) *chosen = best;
   if (table) {

@@ -19,9 +19,9 @@ void check(bool ok, const char* what, long long x = 0, long long y = 0) {
   }
 }
 
-bool packed(jne_context* c, int dim, int64_t n) {
+bool packed(jne_context* c, int dim, int64_t n, int steps = 1000) {
   std::vector<double> out((size_t)n * jne_eigen_count(0, dim));
-  check(jne_eigs_seeded(c, 0, dim, 1000, 1, 1, n, JNE_PREC_MIXED, out.data()) == JNE_OK, "request");
+  check(jne_eigs_seeded(c, 0, dim, steps, 1, 1, n, JNE_PREC_MIXED, out.data()) == JNE_OK, "request");
   return fake::mixed.back().a.pack >= 0;
 }
 
@@ -43,6 +43,9 @@ int main() {
           jne_close(d);
         }
     }
+    for (int steps : {1000 * dim * dim, 1000 * dim * dim + 1, 50000})  // long paths: from 12 runs per SM on
+      for (int64_t n : {12 * fake::kSms, 12 * fake::kSms + 1, 16 * fake::kSms + 1})
+        check(packed(c, dim, n, steps) == (n > (steps > 1000 * dim * dim ? 12 : 16) * fake::kSms), "long paths", steps, n);
     // the tuner: each row times the packing it names; the stored shape leaves the other side of the line to the rule
     for (int64_t n : {line / 2, 8 * line})
       for (bool packed_faster : {false, true}) {

@@ -38,7 +38,7 @@ def test_early_chunk_ends_against_the_general_path(engine, jne, dim, base, seed,
 def test_a_pair_with_an_early_end_keeps_each_runs_bits(engine, jne, dim, base, seed):
     import torch
 
-    line = 12 * torch.cuda.get_device_properties(0).multi_processor_count  # packed above
+    line = 80 * torch.cuda.get_device_properties(0).multi_processor_count  # packed above
     for model in (0, 3, 4):
         alone = {s: engine.eigs_seeded(model, dim, 2100, s, 1, precision=jne.PREC_FP64, base_seed=base)[0]
                  for s in range(seed - 2, seed + 3)}

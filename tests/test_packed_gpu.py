@@ -49,10 +49,10 @@ def test_mixed_packed_against_fp64_and_the_partner(jne, dim, bps):
 @pytest.mark.parametrize("dim", [1, 2, 3, 4])
 @pytest.mark.parametrize("steps", [33, 300, 512, 513, 1100, 2048, 2049, 2500])
 def test_digits_packed(engine, jne, dim, steps):
-    n = 12 * _sms() + 35
+    n = 80 * _sms() + 35  # above the line at every length
     for model in range(5):
-        few = np.concatenate([engine.eigs_seeded(model, dim, steps, 5 + a, min(700, n - a), precision=jne.PREC_FP64)
-                              for a in range(0, n, 700)])
+        few = np.concatenate([engine.eigs_seeded(model, dim, steps, 5 + a, min(1800, n - a), precision=jne.PREC_FP64)
+                              for a in range(0, n, 1800)])
         packed = engine.eigs_seeded(model, dim, steps, 5, n, precision=jne.PREC_FP64)
         assert np.array_equal(packed, few), model
         other = engine.eigs_seeded(model, dim, steps, 6, n - 1, precision=jne.PREC_FP64)  # the other pairs
