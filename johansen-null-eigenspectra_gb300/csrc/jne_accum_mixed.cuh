@@ -435,8 +435,8 @@ __device__ __forceinline__ uint2 product_slot(int t) {
 }
 
 // The product slots' operands of a dim, written by threads `first`, first + stride, ... of those that share the
-// table: a block's warps in the single-request kernels (a table per warp would cost the 6-block variant its sixth
-// block), one warp in the ragged kernel, whose warps may be at different dims.
+// table: a block's warps in the 6-block kernels (a table per warp would cost them their sixth block), one warp in
+// the others (shared by the block, 1 - 2 % slower at dims 2, 4, 5 and 7).
 template <int DIM, bool PACK>
 __device__ __forceinline__ void fill_product_slots(uint2* slot, int first, int stride) {
   constexpr int NU = Packing<DIM, PACK>::kRuns, n = NU * (DIM * (DIM + 1) / 2 + DIM * DIM);
@@ -734,14 +734,21 @@ __global__ void __launch_bounds__(kMixWarps * JNE_WARP, MINB)
     k_accum_mixed(const __grid_constant__ jne_accum_args a, const __grid_constant__ jne_round_keys rk,
                   const __grid_constant__ jne_finalize_args fin) {
   __shared__ WarpSmem sm_all[kMixWarps];
-  __shared__ uint2 slot[kProductSlots];
+  constexpr bool kOwnTable = MINB <= 4;
+  __shared__ uint2 slot_all[kOwnTable ? kMixWarps : 1][kProductSlots];
   // (1 KB of an SM's 228 goes with every block)
-  static_assert(MINB * (sizeof sm_all + sizeof slot + 1024) <= 228 * 1024, "MINB blocks fit an SM's shared memory");
+  static_assert(MINB * (sizeof sm_all + sizeof slot_all + 1024) <= 228 * 1024, "MINB blocks fit an SM's shared memory");
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nwarps = gridDim.x * kMixWarps;
   const bool fused = fin.out != nullptr && a.batch_done != nullptr;
-  fill_product_slots<DIM, PACK>(slot, threadIdx.x, kMixWarps * JNE_WARP);
-  __syncthreads();
+  uint2* slot = slot_all[kOwnTable ? wib : 0];
+  if (kOwnTable) {
+    fill_product_slots<DIM, PACK>(slot, lane, JNE_WARP);
+    __syncwarp();
+  } else {
+    fill_product_slots<DIM, PACK>(slot, threadIdx.x, kMixWarps * JNE_WARP);
+    __syncthreads();
+  }
   const long long units = jne_units(DIM, a.n_runs, PACK);
   auto finalize_done = [&](long long unit) {
     const long long first = batch_complete(a.batch_done, unit, units, lane);
