@@ -49,8 +49,10 @@ extern "C" {
 
 /* arithmetic of the Gram contraction */
 /* plain form: exact Gram sums (digits of the engine's increments on the tensor
- * cores; FP64 multiply-adds for explicit increments and for paths of at most 32
- * steps), FP64 record and solve */
+ * cores, whose FP32 accumulators a chunk's sums exceed with negligible
+ * probability, 9 standard deviations, and are then rounded to FP32; FP64
+ * multiply-adds for explicit increments and for paths of at most 32 steps), FP64
+ * record and solve */
 #define JNE_PREC_FP64 0
 #define JNE_PREC_MIXED 1 /* split FP16/TF32 tensor-core Grams, FP32 chunks, float-float merge, FP64 solve */
 /* JNE_PREC_MIXED requests with fewer steps than this run the FP64 kernel: on
@@ -399,7 +401,7 @@ int jne_simulation_run_models(jne_context* ctx, const char* data_dir, const int*
 int jne_percentiles(const double* eigs, int64_t n, int k, int stat, const double* ps, int np, double* out);
 
 /* The same percentiles of eigenvalues in device memory (n x k, run-major), by
- * a radix select on the device instead of a sort; bit-identical to
+ * a digit select on the device instead of a sort; bit-identical to
  * jne_percentiles.  Work the caller enqueued on `stream` (null: the legacy
  * default stream) before the call is waited for; ps / out are host memory and
  * the call returns when `out` is written.  Scratch: 8 bytes per run within the

@@ -1,5 +1,6 @@
 // jne_accum_digits.cuh -- the plain (FP64) accumulation of the engine's own
-// increments: one warp per run, every Gram sum exact, on the tensor cores.
+// increments: one warp per run (or per pair of runs), every Gram sum exact (as
+// long as it stays in the accumulators' range, below), on the tensor cores.
 //
 // Same contract as jne_accum_f64.cu (rng_matrix.rs:57-141, F's moments of
 // johansen_statistics.rs:102-197 and the sum_of_outer_products calls of
@@ -38,11 +39,12 @@
 // Why: FP64 instructions take 64 cycles a warp and scheduler on this GPU, an
 // m16n8k16 MMA (2048 products) 8.  Dim 12, T 10^4, model 4, 10,000 runs: 50.8 ms
 // with FP64 multiply-adds (one warp per run, 7-9 table entries per lane), 5.78 ms
-// in digits; dim 5, T 1000, 50,001 runs: 9.62 -> 2.07 ms.  Errors against quad
+// in digits; dim 5, T 1000, 50,001 runs: 9.62 -> 1.94 ms.  Errors against quad
 // precision (normwise, rms over runs, dim 12): model 1, T 10^4 2.6e-12 -> 9.3e-15,
 // T 1000 5.5e-14 -> 7.8e-15, T 33 6.2e-15 -> 4.4e-15; shorter paths keep the
 // multiply-adds (jne_accum_digits.cu).
-// What bounds it now: 98 MMAs per 32-step tile (784 cycles), beside which the digit
+// What bounds it now: 94 MMAs per 32-step tile (752 cycles; 2 more for half a tile that
+// has an increment with a fifth digit, about one in 300), beside which the digit
 // extraction's integer instructions (2 cycles each) and the Philox multiplies (3.3)
 // hardly run.  Registers: 72 accumulators; 3 blocks of 4 warps per SM (168
 // registers) measured 5.7 ms of accumulation, 2 blocks (255) 5.8, 4 blocks (128,

@@ -176,9 +176,9 @@ struct jne_accum_args {
   double* mom;               // moment records, SoA
   long long mom_ld;          // leading dimension (>= n_runs)
   unsigned int* status;      // device status word (bit flags), may be null
-  unsigned long long* next_run;  // mixed kernel: zeroed work counter for dynamic run
-                                 // assignment, or null for a fixed stride per warp
-  unsigned int* batch_done;      // mixed kernel with a fused finalize: zeroed count of
+  unsigned long long* next_run;  // zeroed work counter for dynamic run assignment (mixed
+                                 // kernel: or null for a fixed stride per warp)
+  unsigned int* batch_done;      // kernels with a fused finalize: zeroed count of
                                  // accumulated runs per 32-run batch (ceil(n_runs / 32))
   int blocks_per_sm;             // mixed kernel variant: 4 (0 = default) or 6
   int pack;                      // mixed kernel, dims <= 4: >= 0 two runs per warp, < 0 one

@@ -450,7 +450,7 @@ inline int enqueue_seeded(jne_context* c, int model, int dim, int steps, uint64_
   const int k = jne_eigen_count(model, dim);
   uint32_t k0, k1;
   stream_key(base_seed, dim, &k0, &k1);
-  const int64_t per = batch_runs(c, dim, 0) / 2;  // two record buffers in flight
+  const int64_t per = batch_runs(c, dim, 0) / 2;  // two record buffers share the budget (ragged launches use both)
   if (per < 1) return fail(c, JNE_ERR_BUDGET, "budget too small for one run");
   cudaStream_t st = c->stream;
   cudaError_t e = cudaSuccess;

@@ -27,10 +27,11 @@
 // corrections and the unscaled walk (S, S10), rsqrt for sqrt and division, half the
 // rank-two updates, the shift's correction in FP32 (any shift is a valid one: only
 // the convergence depends on it) and the deflation test on exponents.
-// Measured: five models of 40,000 runs at dim 12, T 2000 (one launch for all models
-// included) 11.25 -> 7.70 ms, and 6.9 with QL's sweeps in one loop; 20,011 runs at dim 6,
-// T 100, mostly finalize, 563 -> 447 -> 363 us; errors against quad precision no larger
-// (dim 12, T 100, model 4: 4.1e-14 -> 2.3e-14 rms).
+// Measured, whole calls: five models of 40,000 runs at dim 12, T 2000 (one launch for
+// all models included) 11.25 -> 7.70 ms, 6.9 with QL's sweeps in one loop and 6.63 with
+// two rows of E at a time; 20,011 runs at dim 6, T 100, mostly finalize, 765 -> 413 us.
+// Errors against quad precision are no larger (dim 12, T 100, model 4: 4.1e-14 ->
+// 2.3e-14 rms).
 #pragma once
 #include <cfloat>
 #include <math_constants.h>

@@ -18,7 +18,7 @@
 // the first bins.  Each pass's last block picks the bins and clears the counters, so a
 // pass is one launch; three resolve distinct values, and the host starts more only
 // when they did not.  10^6 x 12, seven percentiles: 444 us before (eight passes of
-// three launches, each comparing every key with every rank's prefix), 130 now, of
+// three launches, each comparing every key with every rank's prefix), 121 now, of
 // which 69 are what a call of 100 rows takes (four launches, a copy and the waits).
 #include <cfloat>
 #include <cstring>
