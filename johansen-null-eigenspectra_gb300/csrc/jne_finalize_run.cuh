@@ -294,9 +294,30 @@ __device__ __noinline__ void finalize_run(const jne_finalize_args& f, int run) {
       }
     }
   }
+  // The reductions square the entries of C.  Explicit increments in FP64 (the separate kernel, lam_scale = T) may put
+  // them where squares overflow or lose bits, beyond 2^400 either way; its diagonal bounds a Gram matrix.  Then an exact
+  // power of two takes C to 1 and the eigenvalues back.
+  int top = 1023 << 20;
+  if (TWO && f.lam_scale != 1.0) {
+    top = 0;
+    for (int p = 0; p < k; p++) top = max(top, exponent_bits(dg[p]));
+  }
+  const bool scaled = TWO && top != 0x7FF00000 && abs(top - (1023 << 20)) > (400 << 20);
+  const int up = min(max((2046 << 20) - top, 1 << 20), 2045 << 20);  // the exponent field of 2^-e, for C of 2^e
+  if (scaled) {
+    const double to_one = __hiloint2double(up, 0);
+    for (int p = 0; p < k; p++) {
+      dg[p] *= to_one;
+      for (int q = p + 1; q < k; q++) S[p][q] *= to_one;
+    }
+  }
   tridiagonalize(S, k, dg, eo);
   if (!tridiagonal_ql(dg, eo, k) && f.status) atomicOr(f.status, JNE_DEV_NOT_SPD);
   for (int j = 0; j < k; j++) dg[j] = fabs(dg[j]) * f.lam_scale;
+  if (scaled) {
+    const double back = __hiloint2double((2046 << 20) - up, 0);
+    for (int j = 0; j < k; j++) dg[j] *= back;
+  }
   for (int j = 1; j < k; j++) {  // insertion sort, descending
     const double v = dg[j];
     int i = j - 1;

@@ -1,5 +1,5 @@
 """Host code of the engine's context on a stand-in CUDA runtime (host memory, recorded launches; no GPU): C++
-checkers compiled here."""
+programs compiled here."""
 import os
 import shutil
 import subprocess

@@ -25,3 +25,18 @@ def test_subnormal_householder_norm(engine, oracle, jne, bits):
         c = 2.0 ** ((bits - np.log2(np.sqrt(r2) * abs(C[0, 1]) + r2)) / 4)  # C scales with c^2, its squares with c^4
         got = engine.eigs_from_increments(0, dB[run:run + 1] * c, precision=jne.PREC_FP64)
         assert normwise_err(got / c / c, ref[run:run + 1]) < 1e-6, run
+
+
+@pytest.mark.parametrize("log2_c", [-480, -300, -264, -256, -250, -201, -200, 200, 201, 250, 254, 256, 300, 480])
+def test_increments_of_any_scale(engine, oracle, jne, log2_c):
+    # S11 scales with c^2, C = E'E and the eigenvalues too: all normal numbers down to c = 2^-480 and up to 2^480, and
+    # for a power of two their bits are those of c = 1 (1e-9: the FP64 tolerance against the oracle)
+    c = 2.0 ** log2_c
+    for dim in (1, 2, 3, 5, 12):
+        for steps in (40, 2000):
+            dB, _ = engine.export_increments(dim, steps, 4, 3)
+            for model in range(5):
+                one = engine.eigs_from_increments(model, dB, precision=jne.PREC_FP64)
+                got = engine.eigs_from_increments(model, dB * c, precision=jne.PREC_FP64)
+                assert normwise_err(got / c / c, one) < 1e-9, (model, dim, steps)
+                assert normwise_err(one, oracle.c_eigs_from_increments(model, dB)) < 1e-9, (model, dim, steps)
