@@ -128,7 +128,7 @@ __device__ __forceinline__ bool tridiagonal_ql(double* dg, double* eo, int n) {
     int m = l;
     for (; l < n; l++, sweeps = 0) {
       // negligible by exponents, with no FP64 instruction: |eo| < eps max(|dg[m]|, |dg[m + 1]|) when it
-      // breaks, within a factor of four of |eo| <= eps (|dg[m]| + |dg[m + 1]|); never for a NaN
+      // breaks, within a factor of four of |eo| <= eps (|dg[m]| + |dg[m + 1]|); never for a NaN eo
       int em = exponent_bits(dg[l]);
       for (m = l; m < n - 1; m++) {
         const int en = exponent_bits(dg[m + 1]);
@@ -312,7 +312,9 @@ __device__ __noinline__ void finalize_run(const jne_finalize_args& f, int run) {
     }
   }
   tridiagonalize(S, k, dg, eo);
-  if (!tridiagonal_ql(dg, eo, k) && f.status) atomicOr(f.status, JNE_DEV_NOT_SPD);
+  // (a single eigenvalue meets no sweep that a NaN or an infinity would keep from converging)
+  const bool good = tridiagonal_ql(dg, eo, k) && !(k == 1 && exponent_bits(dg[0]) == 0x7FF00000);
+  if (!good && f.status) atomicOr(f.status, JNE_DEV_NOT_SPD);
   for (int j = 0; j < k; j++) dg[j] = fabs(dg[j]) * f.lam_scale;
   if (scaled) {
     const double back = __hiloint2double((2046 << 20) - up, 0);

@@ -40,3 +40,17 @@ def test_increments_of_any_scale(engine, oracle, jne, log2_c):
                 got = engine.eigs_from_increments(model, dB * c, precision=jne.PREC_FP64)
                 assert normwise_err(got / c / c, one) < 1e-9, (model, dim, steps)
                 assert normwise_err(one, oracle.c_eigs_from_increments(model, dB)) < 1e-9, (model, dim, steps)
+
+
+@pytest.mark.parametrize("steps", [40, 64, 300, 320])
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_a_single_non_finite_eigenvalue_is_reported(engine, jne, steps, precision):
+    dB, _ = engine.export_increments(1, steps, 4, 2)
+    for bad in (np.nan, np.inf, -np.inf):
+        for step in (0, steps // 2, steps - 1):  # the last increment enters S10 only
+            b = dB.copy()
+            b[1, step, 0] = bad
+            for model in (0, 2, 4):  # one eigenvalue at dim 1
+                with pytest.raises(jne.JneError) as ei:
+                    engine.eigs_from_increments(model, b, precision=precision)
+                assert ei.value.code == jne.JNE_ERR_NUMERIC, (model, bad, step)
