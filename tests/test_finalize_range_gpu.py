@@ -29,8 +29,8 @@ def test_subnormal_householder_norm(engine, oracle, jne, bits):
 
 @pytest.mark.parametrize("log2_c", [-480, -300, -264, -256, -250, -201, -200, 200, 201, 250, 254, 256, 300, 480])
 def test_increments_of_any_scale(engine, oracle, jne, log2_c):
-    # S11 scales with c^2, C = E'E and the eigenvalues too: all normal numbers down to c = 2^-480 and up to 2^480, and
-    # for a power of two their bits are those of c = 1 (1e-9: the FP64 tolerance against the oracle)
+    # S11 scales with c^2, C = E'E and the eigenvalues too, by an exact power of two: all normal numbers down to
+    # c = 2^-480 and up to 2^480 (1e-9: the FP64 tolerance against the oracle)
     c = 2.0 ** log2_c
     for dim in (1, 2, 3, 5, 12):
         for steps in (40, 2000):
